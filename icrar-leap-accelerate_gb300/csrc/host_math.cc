@@ -383,4 +383,122 @@ float grid_table(int32_t C, int32_t taps, double beta, int32_t lbase, int32_t ro
   return static_cast<float>(1.0 / scale);
 }
 
+namespace {
+
+// (hi : lo) with the top bit of hi set and the exponent that keeps the value.
+FxRatio normalised(unsigned __int128 x, int exp) {
+  FxRatio r{0, 0, 0, 0};
+  if (x == 0) return r;
+  while (!(x >> 127)) {
+    x <<= 1;
+    --exp;
+  }
+  r.hi = static_cast<uint64_t>(x >> 64);
+  r.lo = static_cast<uint64_t>(x);
+  r.exp = exp;
+  return r;
+}
+
+// x / c_light to 2^-127 relative, x > 0 (the speed of light is a whole number of metres per second).
+FxRatio over_c(double x) {
+  int e = 0;
+  const double f = std::frexp(x, &e);  // x = f 2^e
+  const uint64_t m = static_cast<uint64_t>(std::ldexp(f, 53)) << 11;  // x = m 2^(e - 64)
+  const uint64_t c = 299792458u;
+  // m 2^160 / c by 32-bit digits: 7 of them, the first of which is 0 or small
+  uint32_t q[7];
+  uint64_t rem = 0;
+  for (int i = 0; i < 7; ++i) {
+    const uint32_t digit = i == 0 ? static_cast<uint32_t>(m >> 32) : i == 1 ? static_cast<uint32_t>(m) : 0u;
+    const uint64_t cur = (rem << 32) | digit;
+    q[i] = static_cast<uint32_t>(cur / c);
+    rem = cur % c;
+  }
+  // x / c = (q[0] .. q[4]) 2^(e - 64 - 96): digits 1..4 as `top`, digit 0 above, digits 5 and 6 below
+  unsigned __int128 top = 0;
+  for (int i = 1; i < 5; ++i) top = (top << 32) | q[i];
+  uint64_t above = q[0], below = (static_cast<uint64_t>(q[5]) << 32) | q[6];
+  int exp = e - 64 - 96 + 128;
+  while (above) {  // shift right until digit 0 is inside the 128 bits
+    below = (below >> 1) | (static_cast<uint64_t>(top & 1) << 63);
+    top = (top >> 1) | (static_cast<unsigned __int128>(above & 1) << 127);
+    above >>= 1;
+    ++exp;
+  }
+  while (top && !(top >> 127)) {
+    top = (top << 1) | (below >> 63);
+    below <<= 1;
+    --exp;
+  }
+  return normalised(top, exp);
+}
+
+// x / (2 pi): the constant is floor(2^128 / pi).
+FxRatio over_two_pi(const FxRatio& x) {
+  if (x.hi == 0) return x;
+  const uint64_t ph = 0x517CC1B727220A94ull, pl = 0xFE13ABE8FA9A6EE0ull;
+  const unsigned __int128 hh = static_cast<unsigned __int128>(x.hi) * ph;
+  const unsigned __int128 mid = (static_cast<unsigned __int128>(x.hi) * pl >> 1) + (static_cast<unsigned __int128>(x.lo) * ph >> 1);
+  return normalised(hh + (mid >> 63), x.exp - 1);
+}
+
+}  // namespace
+
+bool fx_spectrum(double f0, double df, int32_t channels, const double* lambda, FxSpectrum& sp, int32_t* rho) {
+  if (!std::isfinite(f0) || !std::isfinite(df) || !(f0 > 1.0) || f0 > 1e18 || std::fabs(df) > 1e18) return false;
+  double kmax = 0.0;
+  for (int32_t c = 0; c < channels; ++c) {
+    // f0 + c df as an unevaluated sum nh + nl
+    const double p = static_cast<double>(c) * df, pe = std::fma(static_cast<double>(c), df, -p);
+    const double nh = f0 + p, bb = nh - f0, nl = ((f0 - (nh - bb)) + (p - bb)) + pe;
+    if (!(nh > 1.0) || !std::isfinite(nh) || !std::isfinite(lambda[c])) return false;
+    kmax = std::max(kmax, 1.0 / lambda[c]);
+    // lambda (f0 + c df) = c_light + r; 1 / lambda = (f0 + c df) / c_light (1 - r / c_light)
+    const double h = lambda[c] * nh, he = std::fma(lambda[c], nh, -h);
+    const double r = (h - 299792458.0) + he + lambda[c] * nl;
+    const double x = std::nearbyint(std::ldexp(-r / 299792458.0, 64 + kFxFrac));
+    if (!(std::fabs(x) <= static_cast<double>(kFxMaxRho) * (1 << kFxFrac))) return false;
+    rho[c] = static_cast<int32_t>(x);
+  }
+  sp = FxSpectrum{};
+  sp.k0 = over_c(f0);
+  if (df != 0.0) {
+    sp.k1 = over_c(std::fabs(df));
+    sp.kt = over_two_pi(sp.k1);
+  }
+  sp.kmax = kmax * (1.0 + 1e-12);
+  sp.s1 = df < 0 ? -1 : 1;
+  return true;
+}
+
+// cos and sin of the angle x 2^-64 rad, x < 2^64 * pi / 4, in 60-bit fixed point: their Taylor series in whole
+// numbers, each term to 2^-64: the same on every host (long double is software on aarch64: 1.4 ms a context).
+static void fx_cos_sin(uint64_t x, int64_t& c, int64_t& s) {
+  unsigned __int128 term = static_cast<unsigned __int128>(1) << 64;  // x^n / n! in 2^-64
+  __int128 sum[2] = {0, 0};
+  for (int n = 0; term != 0; ++n) {
+    sum[n & 1] += (n & 2) ? -static_cast<__int128>(term) : static_cast<__int128>(term);
+    term = ((term * x) >> 64) / static_cast<unsigned>(n + 1);
+  }
+  c = static_cast<int64_t>((sum[0] + 8) >> 4);
+  s = static_cast<int64_t>((sum[1] + 8) >> 4);
+}
+
+void fx_tables(std::vector<FxLimbs>& out) {
+  out.resize(2 * kFxTable);
+  // 2 pi 2^108: j / 2^10 turns are j (two_pi / 2^10) 2^-108 rad, j / 2^20 turns the same 10 bits further down.
+  const unsigned __int128 two_pi = (static_cast<unsigned __int128>(0x6487ED5110B4ull) << 64) | 0x611A62633145C06Eull;
+  for (int j = 0; j < kFxTable; ++j) {
+    // Quarter turns and the reflection about pi / 4 are exact.
+    const int quad = j / (kFxTable / 4), k = j % (kFxTable / 4);
+    const bool mirror = k > kFxTable / 8;
+    int64_t c, s;
+    fx_cos_sin(static_cast<uint64_t>((two_pi >> 10) * static_cast<unsigned>(mirror ? kFxTable / 4 - k : k) >> 44), c, s);
+    if (mirror) std::swap(c, s);
+    out[j] = quad == 0 ? fx_limbs(c, s) : quad == 1 ? fx_limbs(-s, c) : quad == 2 ? fx_limbs(-c, -s) : fx_limbs(s, -c);
+    fx_cos_sin(static_cast<uint64_t>((two_pi >> 10) * static_cast<unsigned>(j) >> 54), c, s);
+    out[kFxTable + j] = fx_limbs(c, s);
+  }
+}
+
 }  // namespace leapgb

@@ -5,6 +5,8 @@
 #include <string>
 #include <vector>
 
+#include "fixed_phase.h"
+
 namespace leapgb {
 
 // MetaData::GenerateDDMatrix (LA/model/cpu/MetaData.cc:166-203); dd is 3x3 row-major.
@@ -47,5 +49,14 @@ void es_kernel_poly(int32_t taps, double beta, int32_t degree, float* out);
 
 // Psi(k) = integral over |x| < taps/2 of psi(x) cos(2 pi x k / n), for k = 0..kmax.
 std::vector<double> es_kernel_transform(int32_t taps, double beta, int32_t n, int32_t kmax);
+
+// Spectral window of the fixed-point phasors (fixed_phase.h) for channel wavelengths lambda[c],
+// c < channels, as the reference rounds them, and rho[c]: 2^(64 + kFxFrac) times the relative difference of
+// 1 / lambda[c] from (f0 + c df) / c_light.  Returns false where the fixed-point path does not apply:
+// a frequency that is not positive and finite, or wavelengths too far from their own formula.
+bool fx_spectrum(double f0, double df, int32_t channels, const double* lambda, FxSpectrum& sp, int32_t* rho);
+
+// The two phasor tables: kFxTable entries exp(2 pi i j / 2^10), then kFxTable of exp(2 pi i j / 2^20).
+void fx_tables(std::vector<FxLimbs>& out);
 
 }  // namespace leapgb

@@ -4,6 +4,7 @@
 #include "leap_internal.h"
 #include "kernels_solve.cuh"
 #include "kernels_mma.cuh"
+#include "kernels_fixed.cuh"
 
 namespace leapabi {
 
@@ -24,6 +25,43 @@ int dispatch_pols(const RotateArgs& a, dim3 grid, int precision, cudaStream_t s)
     case 4: launch_rotate<VisT, 4>(a, grid, precision, s); return 0;
     default: return -1;
   }
+}
+
+// All-FP64 rotate + average of one item on the integer pipe (kernels_fixed.cuh): the row exponents, then the
+// sums.  nw warps per block take kFxDirs directions each.
+template <typename VisT, int P, int NW>
+int launch_fixed_nw(leap_ctx* ctx, const FxArgs& fa, dim3 grid, cudaStream_t s) {
+  constexpr uint32_t bit = 1u << ((sizeof(VisT) == 8 ? 0 : 9) + (P / 2) * 3 + NW / 2);
+  if (!(ctx->fx_attr_set & bit)) {
+    LEAP_CUDA(cudaFuncSetAttribute(rotate_average_fixed<VisT, P, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   fx_smem_bytes<VisT, P>()),
+              "set shared memory size");
+    ctx->fx_attr_set |= bit;
+  }
+  rotate_average_fixed<VisT, P, NW><<<grid, NW * 32, fx_smem_bytes<VisT, P>(), s>>>(fa);
+  return LEAP_OK;
+}
+
+template <typename VisT, int P>
+int launch_fixed(leap_ctx* ctx, const FxArgs& fa, int nw, dim3 grid, cudaStream_t s) {
+  const int64_t elems = fa.r.rows * P;
+  fx_exponents<VisT><<<static_cast<unsigned>((elems + 31) / 32), 256, 0, s>>>(
+      static_cast<const VisT*>(fa.r.vis), elems, fa.r.channels, const_cast<int16_t*>(fa.vexp));
+  switch (nw) {
+    case 1: return launch_fixed_nw<VisT, P, 1>(ctx, fa, grid, s);
+    case 2: return launch_fixed_nw<VisT, P, 2>(ctx, fa, grid, s);
+    default: return launch_fixed_nw<VisT, P, 4>(ctx, fa, grid, s);
+  }
+}
+
+int dispatch_fixed(leap_ctx* ctx, int32_t vis_type, const FxArgs& fa, int nw, dim3 grid, cudaStream_t s) {
+  if (vis_type == LEAP_VIS_C64)
+    return fa.r.pols == 1 ? launch_fixed<float2, 1>(ctx, fa, nw, grid, s)
+                          : fa.r.pols == 2 ? launch_fixed<float2, 2>(ctx, fa, nw, grid, s)
+                                           : launch_fixed<float2, 4>(ctx, fa, nw, grid, s);
+  return fa.r.pols == 1 ? launch_fixed<double2, 1>(ctx, fa, nw, grid, s)
+                        : fa.r.pols == 2 ? launch_fixed<double2, 2>(ctx, fa, nw, grid, s)
+                                         : launch_fixed<double2, 4>(ctx, fa, nw, grid, s);
 }
 
 // Grid matrix of the gridded kernel for C channels (built once per channel count) and the
@@ -266,6 +304,15 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     LEAP_CUDA(cudaMemcpyAsync(ctx->lambda.ptr, ctx->lambda_host.data(), sizeof(double) * 2 * maxC,
                               cudaMemcpyHostToDevice, s),
               "upload wavelengths");
+    ctx->fx_rho_host.resize(maxC);
+    ctx->fx_ok = fx_spectrum(md.k.freq_start_hz, md.k.freq_inc_hz, maxC, ctx->lambda_host.data(), ctx->fx_sp,
+                             ctx->fx_rho_host.data());
+    if (ctx->fx_ok) {
+      LEAP_CUDA(ctx->fx_rho.ensure(sizeof(int32_t) * maxC), "alloc wavelength corrections");
+      LEAP_CUDA(cudaMemcpyAsync(ctx->fx_rho.ptr, ctx->fx_rho_host.data(), sizeof(int32_t) * maxC,
+                                cudaMemcpyHostToDevice, s),
+                "upload wavelength corrections");
+    }
   }
 
   if (uses_gridded(ctx, items, D, precision, P)) return gridded_stage(ctx, items, d_dd, D, s, kernels);
@@ -441,10 +488,26 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     Integration& in = ctx->integ.at(w.slot);
     const int T = static_cast<int>(in.rows / nbl);
     const int C = in.channels;
-    const int dpw = precision == LEAP_PRECISION_FP64 ? 2 : 4;
-    const int dgroups = (w.ndir + 4 * dpw - 1) / (4 * dpw);
+    const bool fixed = precision == LEAP_PRECISION_FP64 && ctx->fx_ok;
+    int dirs_per_block = precision == LEAP_PRECISION_FP64 ? 8 : 16;  // 4 warps of 2 or 4 directions
+    int nw = 4;
+    if (fixed) {
+      // Warps per block: the split of a stage costs a block about as much as one direction, and directions past
+      // the last one are computed for nothing.
+      int64_t best = std::numeric_limits<int64_t>::max();
+      for (int n : {4, 2, 1}) {
+        const int64_t cost = static_cast<int64_t>((w.ndir + n * kFxDirs - 1) / (n * kFxDirs)) * (n * kFxDirs + 1);
+        if (cost < best) {
+          best = cost;
+          nw = n;
+        }
+      }
+      dirs_per_block = nw * kFxDirs;
+    }
+    const int dgroups = (w.ndir + dirs_per_block - 1) / dirs_per_block;
     int t_per, c_per, nts, ncs;
-    choose_slabs(T, C, static_cast<int64_t>(tiles) * dgroups, t_per, c_per, nts, ncs);
+    if (fixed) choose_fixed_slabs(T, C, static_cast<int64_t>(tiles) * dgroups, ctx->sms * (kFxWarps / nw), t_per, c_per, nts, ncs);
+    else choose_slabs(T, C, static_cast<int64_t>(tiles) * dgroups, t_per, c_per, nts, ncs);
     const int nslab = nts * ncs;
     const int64_t n = static_cast<int64_t>(w.ndir) * P * nbl;
     if (nslab > 1) LEAP_CUDA(ctx->partial.ensure(sizeof(double2) * n * nslab), "alloc partial sums");
@@ -470,10 +533,18 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     double2* avg_item = ctx->avg.as<double2>() + static_cast<int64_t>(w.dir0) * P * nbl;
     ra.out = nslab > 1 ? ctx->partial.as<double2>() : avg_item;
     ra.err = ctx->dev_err.as<int>();
-    const dim3 grid(tiles, dgroups, nslab);
-    int rc = in.vis_type == LEAP_VIS_C64 ? dispatch_pols<float2>(ra, grid, precision, s)
-                                         : dispatch_pols<double2>(ra, grid, precision, s);
-    if (rc != 0) return fail(ctx, LEAP_ERR_INVALID_ARGUMENT, "unsupported polarisation count (1, 2 or 4)");
+    if (fixed) {
+      LEAP_CUDA(ctx->fx_exp.ensure(sizeof(int16_t) * in.rows * P), "alloc row exponents");
+      FxArgs fa{ra, ctx->fx_sp, ctx->fx_tab.as<int4>(), ctx->fx_rho.as<int32_t>(), ctx->fx_exp.as<int16_t>()};
+      const int rc = dispatch_fixed(ctx, in.vis_type, fa, nw, dim3(tiles * dgroups, nslab), s);
+      if (rc != LEAP_OK) return rc;
+      ++kernels;
+    } else {
+      const dim3 grid(tiles, dgroups, nslab);
+      const int rc = in.vis_type == LEAP_VIS_C64 ? dispatch_pols<float2>(ra, grid, precision, s)
+                                                 : dispatch_pols<double2>(ra, grid, precision, s);
+      if (rc != 0) return fail(ctx, LEAP_ERR_INVALID_ARGUMENT, "unsupported polarisation count (1, 2 or 4)");
+    }
     ++kernels;
     if (nslab > 1) {
       reduce_slabs<<<grid_1d(n, 256), 256, 0, s>>>(ctx->partial.as<double2>(), nslab, n, avg_item);

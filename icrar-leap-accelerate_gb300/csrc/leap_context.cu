@@ -96,6 +96,11 @@ int32_t leap_create(int32_t device, leap_ctx** out) {
     LEAP_CUDA(ctx->twiddle_df.ensure(sizeof(float4) * kTwiddleSize), "alloc twiddle table");
     LEAP_CUDA(cudaMemcpy(ctx->twiddle_df.ptr, twd.data(), sizeof(float4) * kTwiddleSize, cudaMemcpyHostToDevice),
               "upload twiddle table");
+    std::vector<FxLimbs> fxt;
+    fx_tables(fxt);
+    LEAP_CUDA(ctx->fx_tab.ensure(sizeof(FxLimbs) * fxt.size()), "alloc phasor tables");
+    LEAP_CUDA(cudaMemcpy(ctx->fx_tab.ptr, fxt.data(), sizeof(FxLimbs) * fxt.size(), cudaMemcpyHostToDevice),
+              "upload phasor tables");
     LEAP_CUDA(ctx->twiddle.ensure(sizeof(float2) * kTwiddleSize), "alloc twiddle table");
     LEAP_CUDA(cudaMemcpy(ctx->twiddle.ptr, tw.data(), sizeof(float2) * kTwiddleSize, cudaMemcpyHostToDevice),
               "upload twiddle table");
@@ -131,6 +136,7 @@ void leap_destroy(leap_ctx* ctx) {
     ctx->dirk.release();
     ctx->twiddle.release();
     ctx->twiddle_df.release();
+    ctx->fx_tab.release(); ctx->fx_rho.release(); ctx->fx_exp.release();
     for (auto& kv : ctx->grid_tabs) kv.second.release();
     ctx->grid_items.release(); ctx->grid_order.release(); ctx->grid_win.release();
     for (auto& tri : ctx->ring)

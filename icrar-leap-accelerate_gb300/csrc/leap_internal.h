@@ -166,6 +166,13 @@ struct leap_ctx {
   int last_ndir = 0, last_pols = 0, last_nbl = 0;
   std::vector<double> lambda_host;
   double lambda_f0 = 0.0, lambda_df = 0.0;
+  // Fixed-point phasors of the all-FP64 form: tables, per-channel corrections, the spectral window
+  // (fx_ok: it applies), and the row exponents of the item being rotated.
+  DeviceBuffer fx_tab, fx_rho, fx_exp;
+  std::vector<int32_t> fx_rho_host;
+  FxSpectrum fx_sp{};
+  bool fx_ok = false;
+  uint32_t fx_attr_set = 0;           // bit per kernel variant whose shared-memory size was raised
   // Ring of (start, after rotate, end) events, one triple per recorded call.
   static constexpr int kRing = 256;
   cudaEvent_t ring[kRing][3] = {};
@@ -236,6 +243,38 @@ inline void choose_slabs_target(int timesteps, int channels, int64_t base_blocks
 // Slab split for the direct-load kernels: about 8 blocks per SM.
 inline void choose_slabs(int timesteps, int channels, int64_t base_blocks, int& t_per, int& c_per, int& nts, int& ncs) {
   choose_slabs_target(timesteps, channels, base_blocks, 152 * 8, t_per, c_per, nts, ncs);
+}
+
+// Slab split for the fixed-point kernel, `resident` of whose blocks run at a time: the fewest slabs whose
+// blocks fill the last round of resident ones to 95%, of whole timesteps, then of 128-channel sums, and of
+// 32-channel blocks (the seeding interval) only where the call is too small to fill the GPU once.
+inline void choose_fixed_slabs(int timesteps, int channels, int64_t base_blocks, int64_t resident, int& t_per, int& c_per,
+                               int& nts, int& ncs) {
+  double best_eff = -1.0;
+  t_per = timesteps; c_per = channels; nts = ncs = 1;
+  for (int unit : {128, 32}) {
+    const int max_c = (channels + unit - 1) / unit;
+    for (int c = 1; c <= max_c; ++c) {
+      const int cp = ((channels + c - 1) / c + unit - 1) / unit * unit;
+      const int cn = (channels + cp - 1) / cp;
+      if (cn != c) continue;
+      for (int t = c == 1 ? 1 : timesteps; t <= std::min(timesteps, 32); ++t) {
+        const int tp = (timesteps + t - 1) / t;
+        const int tn = (timesteps + tp - 1) / tp;
+        // Time of the call in blocks' lengths: rounds of resident blocks times a block's samples.
+        const int64_t blocks = base_blocks * cn * tn;
+        const double rounds = static_cast<double>((blocks + resident - 1) / resident);
+        const double eff = static_cast<double>(base_blocks) * timesteps * channels /
+                           (static_cast<double>(resident) * rounds * tp * std::min(cp, channels));
+        if (eff > best_eff + 0.02) {
+          best_eff = eff;
+          t_per = tp; nts = tn; c_per = cp; ncs = cn;
+        }
+        if (best_eff >= 0.95) return;
+      }
+    }
+    if (best_eff >= 0.5) return;
+  }
 }
 
 // Timestep slabs for the persistent pipelined kernel: the smallest split whose
