@@ -25,16 +25,21 @@
 // Per (row, direction) the phase turns(c) = A + c*B is formed once per
 // timestep in double-float arithmetic (~1e-12 turns) as 32-bit fixed-point
 // fractions of a turn: no FP64 instructions in this kernel (GB300 runs them
-// at ~1/70 of the FP32 rate).  The twiddle is table-accurate (twiddle_turns)
-// every kPipeReseed channels and advanced by one FP32 complex multiply per
-// channel in between (drift over 16 steps ~1e-6; it reaches the cal phases
-// only through baselines that the reference-antenna pass does not cover, with
-// weight ~1/S).  Sums: FP32 over 64 channels, folded into Kahan pairs.
-// Reseeding every 16 rather than 8 channels and folding every 32 rather than 16
-// cut the 128-antenna call from 3.00 to 2.85 ms and moved its cal-phase
-// difference from the FP64 form from 5.5e-7 to 2.1e-6 rad (bar: 1e-5); the
-// paired multiply-accumulate below and folds every 64 then took it to 2.49 ms
-// and 1.6e-6 rad.
+// at ~1/70 of the FP32 rate).  A block of 16 channels is a polynomial in the
+// channel step's phasor w, evaluated by Horner's rule from its last channel:
+//     sum_k V[c0 + k] z w^k = z (V[c0] + w (V[c0+1] + w (...))),
+// so a channel costs one complex multiply-add per pol and no phasor recurrence
+// of its own; z, table-accurate (twiddle_turns), enters once per block.  w has a
+// relative error eta of ~1e-7, w^k one of k eta; z is taken at the block's middle
+// channel and divided by w^8 as rounded, which leaves (k - 8) eta: half the drift
+// of a recurrence from the block's start (~5e-7; it reaches the cal phases only
+// through baselines that the reference-antenna pass does not cover, with weight
+// ~1/S).  Sums: FP32 over 64 channels, folded into Kahan pairs.
+//
+// What bounds it: HBM and the issue of FFMA2, 8 per (row, channel, direction) at
+// 2 to 2.6 issue slots each; a recurrence of the phasors took 4 scalar FMAs more.
+// 32-chunk batched workload, 8 directions a chunk (52.3 GB): 9.6 ms, 5.4 TB/s, in
+// a call of 10.97 -> 10.50 ms.
 //
 // Shared-memory reads: lane i reads its 32 bytes as two 16-byte halves; lanes
 // with bit 2 set read the upper half first so that each quarter-warp covers
@@ -69,7 +74,6 @@ struct PipeParams {
 };
 
 constexpr int kPipeMaxItems = 128;
-constexpr int kPipeReseed = 16;         // channels between table-accurate twiddles
 // Channels summed in FP32 before a Kahan fold.  At 32 the fold was ~6% of the FMA-pipe work;
 // FP32 partial sums over 64 channels (~2e-8 of the sum of |terms|) stay far below the phasor
 // drift between reseeds (~1e-6).  Measured: 32-chunk batched workload 11.47 -> 11.10 ms per
@@ -78,10 +82,11 @@ constexpr int kPipeReseed = 16;         // channels between table-accurate twidd
 constexpr int kPipeFold = 64;
 constexpr int kPipeItemBytes = 32 * 4 * 8;  // one channel of one tile: 32 baselines x 4 pols x complex<float>
 
-// Channels per chunk and ring depth: 1 tile x 16 channels = 16 KB stages, 4 deep; 4 tiles x
-// 16 channels = 64 KB stages, 3 deep (192 KB of the 227 KB of shared memory).
+// Channels per chunk (one Horner block) and ring depth: 1 tile x 16 channels = 16 KB stages, 4 deep; 2 tiles =
+// 32 KB, 4 deep; 4 tiles = 64 KB stages, 3 deep (192 KB of the 227 KB of shared memory).
 template <int TPB> struct PipeShape;
 template <> struct PipeShape<1> { static constexpr int CH = 16, STAGES = 4; };
+template <> struct PipeShape<2> { static constexpr int CH = 16, STAGES = 4; };
 template <> struct PipeShape<4> { static constexpr int CH = 16, STAGES = 3; };
 
 template <int TPB>
@@ -146,33 +151,90 @@ __device__ __forceinline__ void issue_chunk(const ChunkCursor& k, const PipePara
     tma_load_2d(dst + ts * CH * kPipeItemBytes, &it.map, (k.t * p.nbl + (tg * TPB + ts) * 32) * 8, k.cb, &full[st]);
 }
 
-// One channel of the complex multiply-accumulate for DPW directions and 4 pols, on paired
-// FP32 FMAs (FFMA2): each visibility enters as its natural (re, im) register pair v from the
-// shared-memory load and once swapped, vs = (im, re), shared by the DPW directions; the
-// phasor stays a natural (zr, zi) pair advanced by 4 scalar FMAs.  Then
-//     acc_a += v * z = (vr zr, vi zi),   acc_b += vs * z = (vi zr, vr zi),
-// and the fold takes re = acc_a.x - acc_a.y, im = acc_b.x + acc_b.y: 8 paired FMAs (16
-// FMA-pipe cycles) and 4 scalar ones per direction and channel, no per-direction moves.
-template <int DPW>
-__device__ __forceinline__ void mac_channel(const unsigned char* src, int h, float2 (&acc_a)[DPW][4],
-                                            float2 (&acc_b)[DPW][4], float2 (&z)[DPW], const float2 (&w)[DPW]) {
+// Paired FP32 FMAs (FFMA2) run two directions in their halves: a direction pair's phasors and sums are natural
+// register pairs, and a visibility component enters as the addend (v, v).  (With two pols in the halves the
+// step's phasor has to be doubled instead, in moves of every direction: 13.2 against 10.5 ms for the 32-chunk
+// batched workload; scalar FMAs: 12.5 ms.)
+struct PipeStep {  // the phasor w = r + i of a direction pair, and -i
+  float2 r, i, ni;
+};
+
+__device__ __forceinline__ PipeStep pipe_step(float2 r, float2 i) { return PipeStep{r, i, make_float2(-i.x, -i.y)}; }
+
+// p = p * w + v for the 4 pols of one channel and the first N direction pairs: 16 paired FMAs each.  FIRST: p = v.
+template <int N, bool FIRST, int DP>
+__device__ __forceinline__ void pipe_horner(const unsigned char* src, int h, float2 (&pr)[DP][4], float2 (&pi)[DP][4],
+                                            const PipeStep (&w)[DP]) {
   const float4 x0 = *reinterpret_cast<const float4*>(src + 16 * h);
   const float4 x1 = *reinterpret_cast<const float4*>(src + 16 * (1 - h));
-  const float2 v[4] = {make_float2(x0.x, x0.y), make_float2(x0.z, x0.w), make_float2(x1.x, x1.y),
-                       make_float2(x1.z, x1.w)};
-  const float2 vs[4] = {make_float2(x0.y, x0.x), make_float2(x0.w, x0.z), make_float2(x1.y, x1.x),
-                        make_float2(x1.w, x1.z)};
+  const float vr[4] = {x0.x, x0.z, x1.x, x1.z}, vi[4] = {x0.y, x0.w, x1.y, x1.w};
 #pragma unroll
-  for (int j = 0; j < DPW; ++j) {
+  for (int q = 0; q < 4; ++q) {
+    const float2 a = make_float2(vr[q], vr[q]), b = make_float2(vi[q], vi[q]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if (FIRST) {
+        pr[j][q] = a;
+        pi[j][q] = b;
+      } else {
+        const float2 nr = __ffma2_rn(pi[j][q], w[j].ni, __ffma2_rn(pr[j][q], w[j].r, a));
+        pi[j][q] = __ffma2_rn(pr[j][q], w[j].i, __ffma2_rn(pi[j][q], w[j].r, b));
+        pr[j][q] = nr;
+      }
+    }
+  }
+}
+
+// Kahan fold of x into (s, -c): both halves as the scalar sequence y = x - c, t = s + y, c = (t - s) - y, s = t
+// (a - b as fma(b, -1, a), one rounding).
+__device__ __forceinline__ void pipe_fold(float2& s, float2& nc, float2 x) {
+  const float2 neg = make_float2(-1.f, -1.f);
+  const float2 y = __fadd2_rn(x, nc);
+  const float2 t = __fadd2_rn(s, y);
+  nc = __fadd2_rn(y, __ffma2_rn(t, neg, s));
+  s = t;
+}
+
+// acc += z sum_k V[k] w^k over the n channels of a chunk, for the first N direction pairs.  z: the phasor of the
+// chunk's middle channel, at turns a + b (in 2^-32 of a turn) per direction; (ur, ui) = 1 / w^8.
+template <int N, int CH, int DP>
+__device__ __forceinline__ void pipe_chunk(const unsigned char* src, int h, int n, const PipeStep (&w)[DP],
+                                           const float2 (&ur)[DP], const float2 (&ui)[DP], const uint32_t (&turns)[2 * DP],
+                                           const float2* tab, float2 (&acc_r)[DP][4], float2 (&acc_i)[DP][4]) {
+  float2 pr[DP][4], pi[DP][4];
+  pipe_horner<N, true>(src + (n - 1) * kPipeItemBytes, h, pr, pi, w);
+  if (n == CH) {
+#pragma unroll
+    for (int k = CH - 2; k >= 0; --k) pipe_horner<N, false>(src + k * kPipeItemBytes, h, pr, pi, w);
+  } else {
+    for (int k = n - 2; k >= 0; --k) pipe_horner<N, false>(src + k * kPipeItemBytes, h, pr, pi, w);
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    float2 zr, zi;
+    twiddle_turns(turns[2 * j], tab, zr.x, zi.x);
+    twiddle_turns(turns[2 * j + 1], tab, zr.y, zi.y);
+    const float2 nzi = make_float2(-zi.x, -zi.y);
+    const PipeStep x = pipe_step(__ffma2_rn(nzi, ui[j], __fmul2_rn(zr, ur[j])), __ffma2_rn(zi, ur[j], __fmul2_rn(zr, ui[j])));
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      acc_a[j][q] = __ffma2_rn(v[q], z[j], acc_a[j][q]);
-      acc_b[j][q] = __ffma2_rn(vs[q], z[j], acc_b[j][q]);
+      acc_r[j][q] = __ffma2_rn(pi[j][q], x.ni, __ffma2_rn(pr[j][q], x.r, acc_r[j][q]));
+      acc_i[j][q] = __ffma2_rn(pr[j][q], x.i, __ffma2_rn(pi[j][q], x.r, acc_i[j][q]));
     }
-    const float nr = fmaf(z[j].x, w[j].x, -z[j].y * w[j].y);
-    z[j].y = fmaf(z[j].x, w[j].y, z[j].y * w[j].x);
-    z[j].x = nr;
   }
+}
+
+// 1 / w^8 as rounded: conj(w^8) (2 - |w^8|^2), |w^8| = 1 to ~1e-6.
+__device__ __forceinline__ void pipe_unturn8(float wr, float wi, float& ur, float& ui) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float r = fmaf(wr, wr, -wi * wi);
+    wi = 2.f * wr * wi;
+    wr = r;
+  }
+  const float f = 2.f - fmaf(wr, wr, wi * wi);
+  ur = wr * f;
+  ui = -wi * f;
 }
 
 template <int NC, int DPW, int TPB>
@@ -180,7 +242,8 @@ __global__ void __launch_bounds__(NC * 32, 1) rotate_average_mixed_pipe(const Pi
   constexpr int CH = PipeShape<TPB>::CH;
   constexpr int NS = PipeShape<TPB>::STAGES;
   constexpr int WPT = NC / TPB;  // warps (direction groups of DPW) per tile
-  static_assert(NC % TPB == 0, "warps must divide among tiles");
+  constexpr int DP = DPW / 2;    // direction pairs per warp
+  static_assert(NC % TPB == 0 && DPW % 4 == 0, "warps divide among tiles, directions into pairs and halves");
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* stage_mem = smem;
   float2* tab = reinterpret_cast<float2*>(smem + NS * pipe_stage_bytes<TPB>());
@@ -213,7 +276,10 @@ __global__ void __launch_bounds__(NC * 32, 1) rotate_average_mixed_pipe(const Pi
   __syncthreads();
 
   const int h = (lane >> 2) & 1;  // read order of the two 16-byte halves
-  const int ts = warp / WPT, dsub = warp % WPT;
+  // The warps of a tile take its direction groups in an order that differs from tile to tile, so that the groups
+  // past the last direction idle on different schedulers (a warp's scheduler is its number modulo 4).
+  const int ts = warp / WPT;
+  const int dsub = WPT >= 4 ? (warp + 2 * ts) % WPT : (warp + ts / 2) % WPT;
   uint32_t it = 0;
   bool ok = true;
   int item = 0;
@@ -234,12 +300,16 @@ __global__ void __launch_bounds__(NC * 32, 1) rotate_average_mixed_pipe(const Pi
     // A tile wholly past the last baseline (the last tile group when nbl is not a multiple
     // of 32 * TPB) only takes part in the stage hand-over.
     const bool active = jd0 < I.ndir && (tg * TPB + ts) * 32 < p.nbl;
+    // The second half of the warp's directions is past the last one.  Not looked at with 4 tiles, whose items fill
+    // their 8 directions as a rule: the second path costs the full one 1.5% there.
+    const bool half = TPB < 4 && jd0 + DPW / 2 >= I.ndir;
 
-    float sr[DPW][4], si[DPW][4], cr[DPW][4], ci[DPW][4];
+    // Kahan pairs (sum, negated compensation) of direction pair j, pol slot q.
+    float2 sr[DP][4], si[DP][4], cr[DP][4], ci[DP][4];
 #pragma unroll
-    for (int j = 0; j < DPW; ++j)
+    for (int j = 0; j < DP; ++j)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) sr[j][q] = si[j][q] = cr[j][q] = ci[j][q] = 0.f;
+      for (int q = 0; q < 4; ++q) sr[j][q] = si[j][q] = cr[j][q] = ci[j][q] = make_float2(0.f, 0.f);
 
     // The row's split UVWs are loaded one timestep ahead, so that the set-up of a
     // timestep does not wait on a global load.
@@ -249,7 +319,8 @@ __global__ void __launch_bounds__(NC * 32, 1) rotate_average_mixed_pipe(const Pi
       xn[i] = active ? __ldg(I.uvw_f + 6 * (static_cast<int64_t>(t_lo) * p.nbl + (valid ? b : 0)) + i) : 0.f;
     for (int t = t_lo; t < t_hi && ok; ++t) {
       uint32_t pa[DPW], pb[DPW];
-      float2 w[DPW];
+      PipeStep w[DP];
+      float2 ur[DP], ui[DP];  // 1 / w^8
       if (active) {
         // turns(c) = A + c*B, A = -(l*u + m*v + (n-1)*w)*f0/c, B likewise with df.
         float x[6];
@@ -271,18 +342,23 @@ __global__ void __launch_bounds__(NC * 32, 1) rotate_average_mixed_pipe(const Pi
           }
           pa[j] = df_dot3_turns_u32(ka, x);
           pb[j] = df_dot3_turns_u32(kb, x);
-          float wr, wi;
-          twiddle_turns(pb[j], tab, wr, wi);
-          w[j] = make_float2(wr, wi);
+        }
+#pragma unroll
+        for (int j = 0; j < DP; ++j) {
+          float2 r, i;
+          twiddle_turns(pb[2 * j], tab, r.x, i.x);
+          twiddle_turns(pb[2 * j + 1], tab, r.y, i.y);
+          w[j] = pipe_step(r, i);
+          pipe_unturn8(r.x, i.x, ur[j].x, ui[j].x);
+          pipe_unturn8(r.y, i.y, ur[j].y, ui[j].y);
         }
       }
       // FP32 partial sums of up to kPipeFold channels, then a Kahan fold.
-      // acc holds (vr zr, vi zi) and acc_b (vi zr, vr zi) per direction and pol.
-      float2 acc[DPW][4], acc_b[DPW][4];
+      float2 acc_r[DP][4], acc_i[DP][4];
 #pragma unroll
-      for (int j = 0; j < DPW; ++j)
+      for (int j = 0; j < DP; ++j)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[j][q] = acc_b[j][q] = make_float2(0.f, 0.f);
+        for (int q = 0; q < 4; ++q) acc_r[j][q] = acc_i[j][q] = make_float2(0.f, 0.f);
       for (int cb = 0; cb < C; cb += CH, ++it) {
         const int n = min(CH, C - cb);
         const int st = it % NS;
@@ -292,45 +368,22 @@ __global__ void __launch_bounds__(NC * 32, 1) rotate_average_mixed_pipe(const Pi
           break;
         }
         if (active) {
-          float2 z[DPW];
           const unsigned char* src = stage_mem + st * pipe_stage_bytes<TPB>() + ts * CH * kPipeItemBytes + lane * 32;
-          if (n == CH) {
+          uint32_t turns[DPW];
 #pragma unroll
-            for (int sub = 0; sub < CH; sub += kPipeReseed) {
-#pragma unroll
-              for (int j = 0; j < DPW; ++j)
-                twiddle_turns(pa[j] + static_cast<uint32_t>(cb + sub) * pb[j], tab, z[j].x, z[j].y);
-#pragma unroll
-              for (int k = 0; k < kPipeReseed; ++k) {
-                mac_channel<DPW>(src + (sub + k) * kPipeItemBytes, h, acc, acc_b, z, w);
-              }
-            }
-          } else {
-            for (int k = 0; k < n; ++k) {
-              if (k % kPipeReseed == 0) {
-#pragma unroll
-                for (int j = 0; j < DPW; ++j)
-                  twiddle_turns(pa[j] + static_cast<uint32_t>(cb + k) * pb[j], tab, z[j].x, z[j].y);
-              }
-              mac_channel<DPW>(src + k * kPipeItemBytes, h, acc, acc_b, z, w);
-            }
-          }
+          for (int j = 0; j < DPW; ++j) turns[j] = pa[j] + static_cast<uint32_t>(cb + 8) * pb[j];
+          if (half)
+            pipe_chunk<DP / 2, CH>(src, h, n, w, ur, ui, turns, tab, acc_r, acc_i);
+          else
+            pipe_chunk<DP, CH>(src, h, n, w, ur, ui, turns, tab, acc_r, acc_i);
           if ((cb + CH) % kPipeFold == 0 || cb + CH >= C) {
 #pragma unroll
-            for (int j = 0; j < DPW; ++j)
+            for (int j = 0; j < DP; ++j)
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
-                const float re = acc[j][q].x - acc[j][q].y;
-                const float im = acc_b[j][q].x + acc_b[j][q].y;
-                float y = re - cr[j][q];
-                float tt = sr[j][q] + y;
-                cr[j][q] = (tt - sr[j][q]) - y;
-                sr[j][q] = tt;
-                y = im - ci[j][q];
-                tt = si[j][q] + y;
-                ci[j][q] = (tt - si[j][q]) - y;
-                si[j][q] = tt;
-                acc[j][q] = acc_b[j][q] = make_float2(0.f, 0.f);
+                pipe_fold(sr[j][q], cr[j][q], acc_r[j][q]);
+                pipe_fold(si[j][q], ci[j][q], acc_i[j][q]);
+                acc_r[j][q] = acc_i[j][q] = make_float2(0.f, 0.f);
               }
           }
         }
@@ -359,10 +412,11 @@ __global__ void __launch_bounds__(NC * 32, 1) rotate_average_mixed_pipe(const Pi
         if (jd < I.ndir) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const int pol = q ^ (2 * h);
+            const int pol = q ^ (2 * h), i = j >> 1;
+            const bool odd = j & 1;
             out[(static_cast<int64_t>(jd) * 4 + pol) * p.nbl + b] =
-                make_double2(static_cast<double>(sr[j][q]) - static_cast<double>(cr[j][q]),
-                             static_cast<double>(si[j][q]) - static_cast<double>(ci[j][q]));
+                make_double2(static_cast<double>(odd ? sr[i][q].y : sr[i][q].x) + static_cast<double>(odd ? cr[i][q].y : cr[i][q].x),
+                             static_cast<double>(odd ? si[i][q].y : si[i][q].x) + static_cast<double>(odd ? ci[i][q].y : ci[i][q].x));
           }
         }
       }

@@ -270,6 +270,24 @@ bool uses_gridded(const leap_ctx* ctx, const std::vector<WorkItem>& items, int32
   return ctx->gridded == 1 || (ctx->mma_rotate != 2 && min_ndir >= kGridAutoDirs);
 }
 
+// Tiles per block of the pipelined kernel for items of ndir directions.  A block's 8 warps take 4 directions of
+// one tile each, so 4 tiles leave room for 8 directions, 2 for 16 and 1 for 32; fewer tiles than that leave
+// warps idle (128 antennas, 14 timesteps, 384 channels, 9 directions: 0.98 ms a call with 1 tile, 0.69 with 2),
+// more read the visibilities once for each group of directions.
+int pipe_tiles(int ndir) { return ndir <= 8 ? 4 : ndir <= 16 ? 2 : 1; }
+
+template <int TPB>
+int launch_pipe(leap_ctx* ctx, const PipeParams& pp, int grid, cudaStream_t s) {
+  if (!(ctx->pipe_attr_set & TPB)) {
+    LEAP_CUDA(cudaFuncSetAttribute(rotate_average_mixed_pipe<kPipeNC, kPipeDPW, TPB>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, pipe_smem_bytes<TPB>()),
+              "set shared memory size");
+    ctx->pipe_attr_set |= TPB;
+  }
+  rotate_average_mixed_pipe<kPipeNC, kPipeDPW, TPB><<<grid, kPipeNC * 32, pipe_smem_bytes<TPB>(), s>>>(pp);
+  return LEAP_OK;
+}
+
 // Rotate + average of every item into ctx->avg ([D][P][nbl]).
 int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double* d_dd, int32_t D, int32_t precision,
                  int P, cudaStream_t s, int& kernels) {
@@ -318,12 +336,11 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
   if (uses_gridded(ctx, items, D, precision, P)) return gridded_stage(ctx, items, d_dd, D, s, kernels);
   if (all_pipe) {
     // Kernel: the tensor-core one (16 directions per unit) when the autotuner chose it or the
-    // option forces it (items of at least 12 directions); else the CUDA-core one with 4 tiles
-    // per block when items hold at most 8 directions (one block covers 128 baselines x 8
-    // directions), else 1 tile (32 baselines x 32 directions).
+    // option forces it (items of at least 12 directions); else the CUDA-core one with as many tiles
+    // per block as the items' directions leave warps for (pipe_tiles).
     const bool mma = ctx->mma_rotate > 0 && (ctx->tune.mma >= 0 ? ctx->tune.mma == 1
                                                                 : ctx->mma_rotate == 2 && min_ndir >= 12);
-    const int tpb = mma ? 1 : (ctx->tune.tpb > 0) ? ctx->tune.tpb : (min_ndir <= 8 ? 4 : 1);
+    const int tpb = mma ? 1 : ctx->tune.tpb > 0 ? ctx->tune.tpb : pipe_tiles(min_ndir);
     const int wpt = kPipeNC / tpb;
     const int dirs_per_unit = mma ? kMmaDirs : wpt * kPipeDPW;
     const int tgroups = (tiles + tpb - 1) / tpb;
@@ -389,7 +406,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     // steps: timesteps x (padded channels + a per-timestep set-up allowance)).
     const int grid = std::min(units, ctx->sms);
     {
-      const int CH = tpb == 4 ? PipeShape<4>::CH : PipeShape<1>::CH;
+      const int CH = PipeShape<1>::CH;
       std::vector<std::pair<int64_t, int>> cost;
       cost.reserve(units);
       for (const PipeItem& it : pit) {
@@ -454,22 +471,10 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
         ctx->pipe_attr_mma = true;
       }
       rotate_average_mma_pipe<<<grid, kPipeNC * 32, pipe_smem_bytes<1>(), s>>>(pp);
-    } else if (tpb == 4) {
-      if (!ctx->pipe_attr_set4) {
-        LEAP_CUDA(cudaFuncSetAttribute(rotate_average_mixed_pipe<kPipeNC, kPipeDPW, 4>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, pipe_smem_bytes<4>()),
-                  "set shared memory size");
-        ctx->pipe_attr_set4 = true;
-      }
-      rotate_average_mixed_pipe<kPipeNC, kPipeDPW, 4><<<grid, kPipeNC * 32, pipe_smem_bytes<4>(), s>>>(pp);
     } else {
-      if (!ctx->pipe_attr_set) {
-        LEAP_CUDA(cudaFuncSetAttribute(rotate_average_mixed_pipe<kPipeNC, kPipeDPW, 1>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, pipe_smem_bytes<1>()),
-                  "set shared memory size");
-        ctx->pipe_attr_set = true;
-      }
-      rotate_average_mixed_pipe<kPipeNC, kPipeDPW, 1><<<grid, kPipeNC * 32, pipe_smem_bytes<1>(), s>>>(pp);
+      const int rc = tpb == 4 ? launch_pipe<4>(ctx, pp, grid, s) : tpb == 2 ? launch_pipe<2>(ctx, pp, grid, s)
+                                                                             : launch_pipe<1>(ctx, pp, grid, s);
+      if (rc != LEAP_OK) return rc;
     }
     ++kernels;
     if (!red.empty()) {
@@ -883,12 +888,14 @@ std::string batch_key(const leap_ctx* ctx, const std::vector<WorkItem>& items, i
 // events (after one warm-up run) and keep the fastest for this shape.
 int autotune_batch(leap_ctx* ctx, const std::vector<WorkItem>& items, int32_t D, int32_t precision,
                    const std::string& key) {
-  int min_ndir = D;
-  for (const auto& w : items) min_ndir = std::min(min_ndir, w.ndir);
+  int min_ndir = D, max_ndir = 0;
+  for (const auto& w : items) {
+    min_ndir = std::min(min_ndir, w.ndir);
+    max_ndir = std::max(max_ndir, w.ndir);
+  }
   std::vector<TuneChoice> cands;
-  const int tpbs[2] = {1, 4};
-  for (int tpb : tpbs) {
-    if (tpb == 4 && min_ndir > 8) continue;
+  for (int tpb : {pipe_tiles(max_ndir), pipe_tiles(min_ndir)}) {
+    if (!cands.empty() && cands.back().tpb == tpb) continue;
     for (int waves : {2, 4, 8}) cands.push_back(TuneChoice{tpb, waves, 0});
   }
   if (ctx->mma_rotate > 0 && precision == LEAP_PRECISION_MIXED && min_ndir >= 12)

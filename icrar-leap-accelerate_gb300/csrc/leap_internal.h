@@ -107,7 +107,7 @@ using namespace leapabi;
 
 // Launch choices the autotuner may set (0 = built-in heuristic).
 struct TuneChoice {
-  int tpb = 0;    // tiles per block of the pipelined kernel (1 or 4)
+  int tpb = 0;    // tiles per block of the pipelined kernel (1, 2 or 4)
   int waves = 0;  // target rounds of the persistent grid when planning slabs
   int mma = -1;   // 1: tensor-core (mma.sync) bulk kernel, 0: CUDA-core kernel, -1: by direction count
 };
@@ -116,7 +116,7 @@ struct leap_ctx {
   int device = 0;
   int sms = 152;
   bool pageable_direct = false;       // kernels can read pageable host memory in place (ATS / HMM)
-  bool pipe_attr_set = false, pipe_attr_set4 = false;
+  int pipe_attr_set = 0;              // bit per tile count whose shared-memory size was raised
   TuneChoice tune;
   bool capturing = false;             // recording a CUDA graph: skip host-side uploads and timing events
   bool autotune = true;               // tune new batched shapes on first use
