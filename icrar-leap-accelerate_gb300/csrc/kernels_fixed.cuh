@@ -43,6 +43,25 @@ struct FxArgs {
   const int16_t* vexp;    // [rows][pols]: the largest component of the row is below 2^vexp
 };
 
+// A component's magnitude by its bits (the high word of a double): ordered as the magnitudes are, NaN above all.
+__device__ __forceinline__ uint32_t fx_magnitude(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+__device__ __forceinline__ uint32_t fx_magnitude(double x) { return static_cast<uint32_t>(__double2hiint(x)) & 0x7FFFFFFFu; }
+
+// Exponent of the largest magnitude m: it is below 2^e.  kFxPlain where the integer sums do not apply.  m == 0: a
+// row of zeros (or of doubles below 2^-1042), which adds nothing.
+template <typename VisT>
+__device__ __forceinline__ int16_t fx_exponent(uint32_t m) {
+  int e;
+  if (sizeof(VisT) == 8) {
+    const int x = static_cast<int>(m >> 23);
+    e = x == 255 || x < 37 ? kFxPlain : x - 126;  // 2^(28 - e) must be a float
+  } else {
+    const int x = static_cast<int>(m >> 20);
+    e = x == 2047 || x - 1022 > 900 || x - 1022 < -850 ? kFxPlain : x - 1022;  // 2^(e - 56) and its multiples must be doubles
+  }
+  return static_cast<int16_t>(m == 0 ? 0 : e);
+}
+
 // Exponent of each (row, pol): block of 32 elements x 8 channel lanes, reading the cube once.
 template <typename VisT>
 __global__ void __launch_bounds__(256) fx_exponents(const VisT* __restrict__ vis, int64_t elems, int channels,
@@ -50,36 +69,19 @@ __global__ void __launch_bounds__(256) fx_exponents(const VisT* __restrict__ vis
   __shared__ uint32_t part[8][32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int64_t i = blockIdx.x * 32ll + lane;
-  uint32_t m = 0;  // largest magnitude, by its bits (the high word of a double)
+  uint32_t m = 0;
   if (i < elems)
 #pragma unroll 8
     for (int c = g; c < channels; c += 8) {
       const VisT v = __ldg(vis + static_cast<int64_t>(c) * elems + i);
-      if (sizeof(VisT) == 8) {
-        m = max(m, __float_as_uint(static_cast<float>(v.x)) & 0x7FFFFFFFu);
-        m = max(m, __float_as_uint(static_cast<float>(v.y)) & 0x7FFFFFFFu);
-      } else {
-        m = max(m, static_cast<uint32_t>(__double2hiint(static_cast<double>(v.x))) & 0x7FFFFFFFu);
-        m = max(m, static_cast<uint32_t>(__double2hiint(static_cast<double>(v.y))) & 0x7FFFFFFFu);
-      }
+      m = max(m, max(fx_magnitude(v.x), fx_magnitude(v.y)));
     }
   part[g][lane] = m;
   __syncthreads();
   if (g == 0 && i < elems) {
 #pragma unroll
     for (int k = 1; k < 8; ++k) m = max(m, part[k][lane]);
-    int e;
-    if (sizeof(VisT) == 8) {
-      const int x = static_cast<int>(m >> 23);
-      e = x == 255 ? kFxPlain : x - 126;
-      if (m != 0 && e < -90) e = kFxPlain;  // 2^(28 - e) must be a float
-    } else {
-      const int x = static_cast<int>(m >> 20);
-      e = x == 2047 ? kFxPlain : x - 1022;
-      if (e > 960 || (m != 0 && e < -900)) e = kFxPlain;  // 2^(e - 56) and its multiples must be doubles
-    }
-    // An all-zero row (or one of denormals below a double's high word) adds nothing or next to nothing.
-    out[i] = static_cast<int16_t>(m == 0 ? 0 : e);
+    out[i] = fx_exponent<VisT>(m);
   }
 }
 
@@ -324,6 +326,54 @@ __device__ __forceinline__ FxLimbs fx_lookup(const int4* tab, uint64_t t) {
   return fx_turn(t, FxLimbs{a.x, a.y, a.z, a.w}, FxLimbs{b.x, b.y, b.z, b.w});
 }
 
+// The phasor of one (row, direction), channel by channel.
+struct FxRay {
+  FxPhase ph;
+  FxLimbs w;        // channel step; 0 for a row that does not fit
+  int64_t zr, zi;   // 60-bit phasor
+
+  // At channel c0 of a row.  Returns whether sf fits; if not, the phasor is 0.
+  __device__ __forceinline__ bool begin(double sf, const FxSpectrum& sp, int c0, const int4* tab) {
+    const bool fits = fx_in_range(sf, sp);
+    uint64_t step;
+    fx_setup(ph, fits ? sf : 0.0, sp, c0, step);
+    w = fx_lookup(tab, step);
+    if (!fits) w = FxLimbs{0, 0, 0, 0};
+    return fits;
+  }
+  __device__ __forceinline__ void seed(int32_t rho, const int4* tab) {
+    ph.e = fx_residual(ph, rho);
+    const FxLimbs z = fx_lookup(tab, fx_turns(ph));
+    const bool fits = w.rh != 0 || w.ih != 0;  // a phasor's high limbs are not both 0
+    zr = fits ? (static_cast<int64_t>(z.rh) << 30) + z.rl : 0;
+    zi = fits ? (static_cast<int64_t>(z.ih) << 30) + z.il : 0;
+  }
+  __device__ __forceinline__ void next(int32_t rho) { fx_step(zr, zi, w, fx_advance(ph, rho)); }
+};
+
+// sf = -2 pi (w_rot - w) of a row, without fused operations, as the reference forms it.
+__device__ __forceinline__ double fx_shift_factor(const double* dd2, double u, double v, double w) {
+  const double wrot = __dadd_rn(__dadd_rn(__dmul_rn(__ldg(dd2), u), __dmul_rn(__ldg(dd2 + 1), v)), __dmul_rn(__ldg(dd2 + 2), w));
+  return __dmul_rn(-kTwoPi, __dadd_rn(wrot, -w));
+}
+
+// Fetch of channels [c0, c0 + n) of the 32 rows from r0 (rows >= nrows of them are zero) to raw, by all threads of
+// the block: pieces of 16 bytes (8 for a single complex<float>), lanes along a channel's rows.
+template <typename VisT, int P>
+__device__ __forceinline__ void fx_fetch(unsigned char* raw, const void* vis, int64_t rows, int64_t r0, int nrows, int c0, int n) {
+  constexpr int kGroup = P * static_cast<int>(sizeof(VisT));
+  constexpr int kPiece = kGroup >= 16 ? 16 : 8;
+  constexpr int kPieces = kGroup * 32 / kPiece;  // per channel
+  const char* base = static_cast<const char*>(vis);
+  for (int i = threadIdx.x; i < n * kPieces; i += blockDim.x) {
+    const int k = i / kPieces, q = i % kPieces;
+    const bool ok = q * kPiece / kGroup < nrows;
+    const int64_t off = (static_cast<int64_t>(c0 + k) * rows + r0) * kGroup + q * kPiece;
+    fx_copy_async(raw + (k * kPieces + q) * kPiece, base + (ok ? off : 0), ok, kPiece);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 // A block is NW warps of kFxDirs directions each, over 32 baselines (one per lane) and a slab of timesteps
 // and channels.  The raw visibilities of a stage (kFxStage channels) arrive by cp.async while the previous
 // stage computes; all warps split them into limbs once, and every warp reads the limbs.
@@ -348,29 +398,14 @@ __global__ void __launch_bounds__(NW * 32, kFxWarps / NW) rotate_average_fixed(c
   const int nst = (c_hi - c_lo + kFxStage - 1) / kFxStage;  // stages per timestep
   const int total = (t_hi - t_lo) * nst;
 
-  // Pieces of a stage: 16 bytes (8 for a single complex<float>), lanes along a channel's rows.
-  constexpr int kPiece = P * static_cast<int>(sizeof(VisT)) >= 16 ? 16 : 8;
-  constexpr int kPieces = P * static_cast<int>(sizeof(VisT)) * 32 / kPiece;  // per channel of the tile
   auto fetch = [&](int s) {
     const int t = t_lo + s / nst, c0 = c_lo + (s % nst) * kFxStage;
-    const int n = min(kFxStage, c_hi - c0);
-    const char* base = static_cast<const char*>(ra.vis);
-    for (int i = threadIdx.x; i < n * kPieces; i += NW * 32) {
-      const int k = i / kPieces, q = i % kPieces;
-      const int row = q * kPiece / (P * static_cast<int>(sizeof(VisT)));
-      const bool ok = b0 + row < ra.nbl;
-      const int64_t off = ((static_cast<int64_t>(c0 + k) * ra.rows + static_cast<int64_t>(t) * ra.nbl + b0) * P) *
-                              static_cast<int64_t>(sizeof(VisT)) + q * kPiece;
-      fx_copy_async(fx_smem + (k * kPieces + q) * kPiece, base + (ok ? off : 0), ok, kPiece);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    fx_fetch<VisT, P>(fx_smem, ra.vis, ra.rows, static_cast<int64_t>(t) * ra.nbl + b0, ra.nbl - b0, c0, min(kFxStage, c_hi - c0));
   };
 
   double sum[kFxDirs][P][2];
   Sum acc[kFxDirs];
-  FxPhase ph[kFxDirs];
-  FxLimbs w[kFxDirs];
-  int64_t zr[kFxDirs], zi[kFxDirs];  // 60-bit phasors
+  FxRay ray[kFxDirs];
   int ve[P];
 #pragma unroll
   for (int j = 0; j < kFxDirs; ++j)
@@ -405,14 +440,8 @@ __global__ void __launch_bounds__(NW * 32, kFxWarps / NW) rotate_average_fixed(c
       const double u = __ldg(ra.uvw + 3 * r), v = __ldg(ra.uvw + 3 * r + 1), x = __ldg(ra.uvw + 3 * r + 2);
 #pragma unroll
       for (int j = 0; j < kFxDirs; ++j) {
-        const double* dd = ra.dd + 9 * min(d0 + j, ra.ndir - 1) + 6;
-        const double wrot = __dadd_rn(__dadd_rn(__dmul_rn(__ldg(dd), u), __dmul_rn(__ldg(dd + 1), v)), __dmul_rn(__ldg(dd + 2), x));
-        const double sf = __dmul_rn(-kTwoPi, __dadd_rn(wrot, -x));
-        const bool fits = fx_in_range(sf, a.sp);
-        uint64_t step;
-        fx_setup(ph[j], fits ? sf : 0.0, a.sp, c_lo, step);
-        w[j] = fx_lookup(a.tab, step);
-        if (!fits) w[j] = FxLimbs{0, 0, 0, 0};  // (with zr = zi = 0) nothing from the integer sums
+        const double sf = fx_shift_factor(ra.dd + 9 * min(d0 + j, ra.ndir - 1) + 6, u, v, x);
+        const bool fits = ray[j].begin(sf, a.sp, c_lo, a.tab);
         if (valid && (plain_row || !fits)) {
           double2 add[P];
           fx_plain_row<VisT, P>(ra, r, sf, c_lo, c_hi, add);
@@ -426,13 +455,7 @@ __global__ void __launch_bounds__(NW * 32, kFxWarps / NW) rotate_average_fixed(c
     }
     if (cf % kFxSeed == 0) {
 #pragma unroll
-      for (int j = 0; j < kFxDirs; ++j) {
-        ph[j].e = fx_residual(ph[j], __ldg(a.rho + cb));
-        const FxLimbs z = fx_lookup(a.tab, fx_turns(ph[j]));
-        const bool fits = w[j].rh != 0 || w[j].ih != 0;  // a phasor's high limbs are not both 0
-        zr[j] = fits ? (static_cast<int64_t>(z.rh) << 30) + z.rl : 0;
-        zi[j] = fits ? (static_cast<int64_t>(z.ih) << 30) + z.il : 0;
-      }
+      for (int j = 0; j < kFxDirs; ++j) ray[j].seed(__ldg(a.rho + cb), a.tab);
     }
     if (cf % Sum::kFlush == 0) {
 #pragma unroll
@@ -444,8 +467,8 @@ __global__ void __launch_bounds__(NW * 32, kFxWarps / NW) rotate_average_fixed(c
       const typename Sum::Vis v = Sum::load(limb, k, lane);
 #pragma unroll
       for (int j = 0; j < kFxDirs; ++j) {
-        acc[j].add(v, Sum::phasor(zr[j], zi[j]));
-        fx_step(zr[j], zi[j], w[j], fx_advance(ph[j], rho));
+        acc[j].add(v, Sum::phasor(ray[j].zr, ray[j].zi));
+        ray[j].next(rho);
       }
     }
     if ((cf + kFxStage) % Sum::kFlush == 0 || cb + kFxStage >= c_hi) {

@@ -3,6 +3,48 @@
 #include "kernels_solve.cuh"
 #include "kernels_adjoint.cuh"
 
+namespace leapabi {
+
+// Rotate + average adjoint in fixed point: dL/d(l, m, n) to d_grad_lmn and, with aa.gvis, dL/dV.
+template <typename VisT, int P, int NW>
+int launch_adjoint_lmn(leap_ctx* ctx, const AdjointFixedArgs& fa, dim3 grid, cudaStream_t s) {
+  constexpr int smem = fx_raw_bytes<VisT, P>() + kFxStage * 32 * 16;
+  LEAP_CUDA(cudaFuncSetAttribute(adjoint_lmn_fixed<VisT, P, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+            "set shared memory size");
+  adjoint_lmn_fixed<VisT, P, NW><<<grid, NW * 32, smem, s>>>(fa);
+  return LEAP_OK;
+}
+
+template <typename VisT, int P>
+int adjoint_fixed(leap_ctx* ctx, AdjointFixedArgs fa, double* d_grad_lmn, cudaStream_t s) {
+  const AdjointArgs& a = fa.a;
+  const int nbl = a.nbl, D = a.D;
+  // Up to 16 directions a block (the split of a stage into limbs is done once for them); fewer, and channel or
+  // timestep slabs, as the forward kernel has them.
+  const int nw = D <= 2 ? 1 : D <= 4 ? 2 : D <= 8 ? 4 : 8;
+  const int tiles = (nbl + 31) / 32, dgroups = (D + nw * kFxDirs - 1) / (nw * kFxDirs);
+  choose_fixed_slabs(fa.T, a.C, static_cast<int64_t>(tiles) * dgroups, ctx->sms * (16 / nw), fa.t_per_slab, fa.c_per_slab,
+                     fa.n_tslab, fa.n_cslab);
+  const int nslab = fa.n_tslab * fa.n_cslab, nblk = tiles * nslab;
+  LEAP_CUDA(ctx->adj_partial.ensure(sizeof(double) * 3 * static_cast<size_t>(nblk) * D), "alloc adjoint partials");
+  fa.a.partial = ctx->adj_partial.as<double>();
+  adjoint_exponents<VisT, P><<<static_cast<unsigned>((a.rows + 31) / 32), 256, 0, s>>>(
+      static_cast<const VisT*>(a.vis), a.rows, a.C, a.check_nan, const_cast<int16_t*>(fa.vexp));
+  const dim3 grid(tiles * dgroups, nslab);
+  const int rc = nw == 1 ? launch_adjoint_lmn<VisT, P, 1>(ctx, fa, grid, s) : nw == 2 ? launch_adjoint_lmn<VisT, P, 2>(ctx, fa, grid, s)
+               : nw == 4 ? launch_adjoint_lmn<VisT, P, 4>(ctx, fa, grid, s) : launch_adjoint_lmn<VisT, P, 8>(ctx, fa, grid, s);
+  if (rc != LEAP_OK) return rc;
+  adjoint_lmn_reduce<<<(3 * D + 3) / 4, 128, 0, s>>>(fa.a.partial, nblk, D, d_grad_lmn);
+  if (a.gvis) {
+    adjoint_split_g<<<(nbl + 127) / 128, 128, 0, s>>>(a.gavg, nbl, D, const_cast<int4*>(fa.g), const_cast<int16_t*>(fa.gexp));
+    const int64_t units = ((a.rows + 31) / 32) * ((a.C + kVisChannels - 1) / kVisChannels);
+    adjoint_vis_fixed<VisT, P><<<static_cast<unsigned>((units + 3) / 4), 128, 0, s>>>(fa);
+  }
+  return LEAP_OK;
+}
+
+}  // namespace leapabi
+
 extern "C" {
 
 int32_t leap_backward(leap_ctx* ctx, int32_t slot, const double* d_dd, int32_t ndir, const double* d_avg0,
@@ -30,9 +72,9 @@ int32_t leap_backward(leap_ctx* ctx, int32_t slot, const double* d_dd, int32_t n
                                                              ctx->adj_dphi.as<double>(), nI);
   else
     LEAP_CUDA(cudaMemsetAsync(ctx->adj_dphi.ptr, 0, sizeof(double) * D, s), "clear");
-  adjoint_cal1<<<(S * D + 255) / 256, 256, 0, s>>>(d_grad_cal, ctx->adj_dphi.as<double>(), std::max(nI, 1),
-                                                   md.at_ptr.as<int32_t>(), md.at_idx.as<int32_t>(),
-                                                   md.at_val.as<double>(), S, D, ctx->adj_cal1.as<double>());
+  adjoint_cal1<<<static_cast<unsigned>((static_cast<int64_t>(S) * D * 32 + 255) / 256), 256, 0, s>>>(
+      d_grad_cal, ctx->adj_dphi.as<double>(), std::max(nI, 1), md.at_ptr.as<int32_t>(), md.at_idx.as<int32_t>(),
+      md.at_val.as<double>(), S, D, ctx->adj_cal1.as<double>());
   if (nI1 > 0)
     adjoint_contract_t<<<(nI1 * 32 + 255) / 256, 256, 0, s>>>(md.Ad1.as<double>(), S, nI1, ctx->adj_cal1.as<double>(),
                                                               D, ctx->adj_phi1.as<double>(), nI1);
@@ -40,8 +82,8 @@ int32_t leap_backward(leap_ctx* ctx, int32_t slot, const double* d_dd, int32_t n
   adjoint_avg_dint<<<grid_1d(static_cast<int64_t>(nbl) * D, 256), 256, 0, s>>>(
       avg0, ctx->adj_dphi.as<double>(), std::max(nI, 1), nI, nbl, D, ctx->adj_gavg.as<double2>());
   if (nI1 > 0)
-    adjoint_avg_phi1<<<(D + 127) / 128, 128, 0, s>>>(avg0, ctx->adj_phi1.as<double>(), md.I1.as<int32_t>(), nI1, nbl,
-                                                     D, ctx->adj_gavg.as<double2>());
+    adjoint_avg_phi1<<<D, 256, 0, s>>>(avg0, ctx->adj_phi1.as<double>(), md.I1.as<int32_t>(), nI1, nbl, D,
+                                       ctx->adj_gavg.as<double2>());
   // Rotate + average adjoint over the integration, recomputing the rotated samples.
   AdjointArgs aa{};
   aa.vis = d_vis ? d_vis : in.vis.ptr;
@@ -57,6 +99,42 @@ int32_t leap_backward(leap_ctx* ctx, int32_t slot, const double* d_dd, int32_t n
   aa.D = D;
   aa.f0 = md.k.freq_start_hz;
   aa.df = md.k.freq_inc_hz;
+  {
+    const int rc = ensure_spectrum(ctx, aa.C, s);
+    if (rc != LEAP_OK) return rc;
+  }
+  aa.gvis = d_grad_vis;
+  // The fixed-point kernels read and write 16-byte pieces (8 for a single complex<float>); arrays that are not
+  // aligned to that, and spectral windows that fixed_phase.h does not take, use the FP64 ones.
+  const size_t esz = aa.vis_c64 ? sizeof(float2) : sizeof(double2);
+  const uintptr_t align = esz * aa.P % 16 == 0 ? 16 : 8;
+  if (ctx->fx_ok && in.rows % nbl == 0 && (reinterpret_cast<uintptr_t>(aa.vis) | reinterpret_cast<uintptr_t>(d_grad_vis)) % align == 0) {
+    LEAP_CUDA(ctx->fx_exp.ensure(sizeof(int16_t) * in.rows), "alloc row exponents");
+    LEAP_CUDA(ctx->adj_g.ensure(sizeof(int4) * static_cast<size_t>(nbl) * D), "alloc adjoint scratch");
+    LEAP_CUDA(ctx->adj_gexp.ensure(sizeof(int16_t) * nbl), "alloc adjoint scratch");
+    AdjointFixedArgs fa{};
+    fa.a = aa;
+    fa.sp = ctx->fx_sp;
+    fa.tab = ctx->fx_tab.as<int4>();
+    fa.rho = ctx->fx_rho.as<int32_t>();
+    fa.lambda = ctx->lambda.as<double>();
+    fa.inv_lambda = ctx->lambda.as<double>() + ctx->lambda_host.size() / 2;
+    fa.vexp = ctx->fx_exp.as<int16_t>();
+    fa.kexp = std::ilogb(ctx->fx_sp.kmax) + 1;
+    fa.T = static_cast<int>(in.rows / nbl);
+    fa.g = ctx->adj_g.as<int4>();
+    fa.gexp = ctx->adj_gexp.as<int16_t>();
+    int rc = LEAP_OK;
+    if (aa.vis_c64)
+      rc = aa.P == 1 ? adjoint_fixed<float2, 1>(ctx, fa, d_grad_lmn, s) : aa.P == 2 ? adjoint_fixed<float2, 2>(ctx, fa, d_grad_lmn, s)
+                                                                                    : adjoint_fixed<float2, 4>(ctx, fa, d_grad_lmn, s);
+    else
+      rc = aa.P == 1 ? adjoint_fixed<double2, 1>(ctx, fa, d_grad_lmn, s) : aa.P == 2 ? adjoint_fixed<double2, 2>(ctx, fa, d_grad_lmn, s)
+                                                                                     : adjoint_fixed<double2, 4>(ctx, fa, d_grad_lmn, s);
+    if (rc != LEAP_OK) return rc;
+    LEAP_CUDA(cudaGetLastError(), "adjoint launch");
+    return LEAP_OK;
+  }
   constexpr int kDPB = 4;
   const int64_t items = in.rows * ((in.channels + kAdjChannels - 1) / kAdjChannels);
   const int dgroups = (D + kDPB - 1) / kDPB;
@@ -65,12 +143,10 @@ int32_t leap_backward(leap_ctx* ctx, int32_t slot, const double* d_dd, int32_t n
   LEAP_CUDA(ctx->adj_partial.ensure(sizeof(double) * 3 * static_cast<size_t>(bx) * D), "alloc adjoint partials");
   aa.partial = ctx->adj_partial.as<double>();
   adjoint_lmn<kDPB><<<dim3(bx, dgroups), 256, 0, s>>>(aa);
-  adjoint_lmn_reduce<<<(3 * D + 127) / 128, 128, 0, s>>>(aa.partial, bx, D, d_grad_lmn);
+  adjoint_lmn_reduce<<<(3 * D + 3) / 4, 128, 0, s>>>(aa.partial, bx, D, d_grad_lmn);
   if (d_grad_vis) {
-    const size_t esz = aa.vis_c64 ? sizeof(float2) : sizeof(double2);
     LEAP_CUDA(cudaMemsetAsync(d_grad_vis, 0, esz * static_cast<size_t>(in.rows) * in.channels * in.pols, s),
               "clear vis gradient");
-    aa.gvis = d_grad_vis;
     adjoint_vis<<<grid_1d(items, 256), 256, 0, s>>>(aa);
   }
   LEAP_CUDA(cudaGetLastError(), "adjoint launch");

@@ -288,6 +288,40 @@ int launch_pipe(leap_ctx* ctx, const PipeParams& pp, int grid, cudaStream_t s) {
   return LEAP_OK;
 }
 
+// Channel wavelengths of at least `channels` channels, computed exactly as Constants::GetChannelWavelength does, and
+// the fixed-point spectral window; uploaded only when the channel count or the spectral window changes.
+int ensure_spectrum(leap_ctx* ctx, int channels, cudaStream_t s) {
+  const Metadata& md = ctx->md;
+  LEAP_CUDA(ctx->lambda.ensure(sizeof(double) * 2 * channels), "alloc wavelengths");
+  if (ctx->lambda_host.size() != static_cast<size_t>(2 * channels) || ctx->lambda_f0 != md.k.freq_start_hz ||
+      ctx->lambda_df != md.k.freq_inc_hz) {
+    // [wavelengths][their reciprocals]: c / (f0 + ch*df) with each operation rounded on its own,
+    // as the reference's Constants::GetChannelWavelength (no fused multiply-add).
+    ctx->lambda_host.resize(2 * channels);
+    for (int c = 0; c < channels; ++c) {
+      volatile double prod = static_cast<double>(c) * md.k.freq_inc_hz;
+      const double lam = kSpeedOfLight / (md.k.freq_start_hz + prod);
+      ctx->lambda_host[c] = lam;
+      ctx->lambda_host[channels + c] = 1.0 / lam;
+    }
+    ctx->lambda_f0 = md.k.freq_start_hz;
+    ctx->lambda_df = md.k.freq_inc_hz;
+    LEAP_CUDA(cudaMemcpyAsync(ctx->lambda.ptr, ctx->lambda_host.data(), sizeof(double) * 2 * channels,
+                              cudaMemcpyHostToDevice, s),
+              "upload wavelengths");
+    ctx->fx_rho_host.resize(channels);
+    ctx->fx_ok = fx_spectrum(md.k.freq_start_hz, md.k.freq_inc_hz, channels, ctx->lambda_host.data(), ctx->fx_sp,
+                             ctx->fx_rho_host.data());
+    if (ctx->fx_ok) {
+      LEAP_CUDA(ctx->fx_rho.ensure(sizeof(int32_t) * channels), "alloc wavelength corrections");
+      LEAP_CUDA(cudaMemcpyAsync(ctx->fx_rho.ptr, ctx->fx_rho_host.data(), sizeof(int32_t) * channels,
+                                cudaMemcpyHostToDevice, s),
+                "upload wavelength corrections");
+    }
+  }
+  return LEAP_OK;
+}
+
 // Rotate + average of every item into ctx->avg ([D][P][nbl]).
 int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double* d_dd, int32_t D, int32_t precision,
                  int P, cudaStream_t s, int& kernels) {
@@ -303,34 +337,9 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     maxC = std::max(maxC, in.channels);
     min_ndir = std::min(min_ndir, w.ndir);
   }
-  // Channel wavelengths, computed exactly as Constants::GetChannelWavelength does;
-  // uploaded only when the channel count or the spectral window changes.
-  LEAP_CUDA(ctx->lambda.ensure(sizeof(double) * 2 * maxC), "alloc wavelengths");
-  if (ctx->lambda_host.size() != static_cast<size_t>(2 * maxC) || ctx->lambda_f0 != md.k.freq_start_hz ||
-      ctx->lambda_df != md.k.freq_inc_hz) {
-    // [wavelengths][their reciprocals]: c / (f0 + ch*df) with each operation rounded on its own,
-    // as the reference's Constants::GetChannelWavelength (no fused multiply-add).
-    ctx->lambda_host.resize(2 * maxC);
-    for (int c = 0; c < maxC; ++c) {
-      volatile double prod = static_cast<double>(c) * md.k.freq_inc_hz;
-      const double lam = kSpeedOfLight / (md.k.freq_start_hz + prod);
-      ctx->lambda_host[c] = lam;
-      ctx->lambda_host[maxC + c] = 1.0 / lam;
-    }
-    ctx->lambda_f0 = md.k.freq_start_hz;
-    ctx->lambda_df = md.k.freq_inc_hz;
-    LEAP_CUDA(cudaMemcpyAsync(ctx->lambda.ptr, ctx->lambda_host.data(), sizeof(double) * 2 * maxC,
-                              cudaMemcpyHostToDevice, s),
-              "upload wavelengths");
-    ctx->fx_rho_host.resize(maxC);
-    ctx->fx_ok = fx_spectrum(md.k.freq_start_hz, md.k.freq_inc_hz, maxC, ctx->lambda_host.data(), ctx->fx_sp,
-                             ctx->fx_rho_host.data());
-    if (ctx->fx_ok) {
-      LEAP_CUDA(ctx->fx_rho.ensure(sizeof(int32_t) * maxC), "alloc wavelength corrections");
-      LEAP_CUDA(cudaMemcpyAsync(ctx->fx_rho.ptr, ctx->fx_rho_host.data(), sizeof(int32_t) * maxC,
-                                cudaMemcpyHostToDevice, s),
-                "upload wavelength corrections");
-    }
+  {
+    const int rc = ensure_spectrum(ctx, maxC, s);
+    if (rc != LEAP_OK) return rc;
   }
 
   if (uses_gridded(ctx, items, D, precision, P)) return gridded_stage(ctx, items, d_dd, D, s, kernels);

@@ -162,7 +162,7 @@ void leap_destroy(leap_ctx* ctx) {
     ctx->refant_items.release();
     ctx->refant_reduce.release();
     ctx->adj_dphi.release(); ctx->adj_cal1.release(); ctx->adj_phi1.release(); ctx->adj_gavg.release();
-    ctx->adj_partial.release();
+    ctx->adj_partial.release(); ctx->adj_g.release(); ctx->adj_gexp.release();
     ctx->flag_count.release();
     for (int b = 0; b < 2; ++b) {
       ctx->stage_dev[b].release();

@@ -135,7 +135,7 @@ struct leap_ctx {
   bool pipe_attr_mma = false;
   int tc_attr_set = 0;                // bit per N tile whose shared-memory size was raised
   DeviceBuffer dphi_tc;               // packed dphi operand of the tensor-core contraction
-  DeviceBuffer adj_dphi, adj_cal1, adj_phi1, adj_gavg, adj_partial;  // adjoint scratch
+  DeviceBuffer adj_dphi, adj_cal1, adj_phi1, adj_gavg, adj_partial, adj_g, adj_gexp;  // adjoint scratch
   DeviceBuffer flag_count;
   // MeasurementSet-order ingestion from pageable host memory: two pinned staging
   // buffers and their device twins, each reused once its piece has been transposed.
@@ -309,5 +309,6 @@ int fill_timings(leap_ctx* ctx, leap_timings* out);
 void finish_upload(Integration& in);
 // Defined in leap_calibrate.cu.
 void wait_for_uploads(leap_ctx* ctx, const std::vector<WorkItem>& items, cudaStream_t s);
+int ensure_spectrum(leap_ctx* ctx, int channels, cudaStream_t s);
 
 }  // namespace leapabi
