@@ -145,56 +145,91 @@ __host__ __device__ constexpr int grid_f16_offset(int row, int k) {
   return ((row >> 3) * 2 + (k >> 3)) * 128 + (row & 7) * 16 + (k & 7) * 2;
 }
 
-// Builds the split grid operand of a 4-pol complex<float> integration [C][rows][8 floats]:
-// one 128-thread block per (quad, timestep block); warp w takes timestep w of the block and
-// lane = 8 q + 2 p + s, the baseline q of the quad, pol p, (re, im) s.  The power of two
-// of each (baseline, pol) brings its largest |component| over the block's 4 timesteps and
-// all channels into [2^13, 2^14); vinv holds its inverse (1 for an all-zero one).  hi is
-// the scaled visibility rounded to FP16, lo the remainder rounded to FP16.  Rows and
-// channels past the integration are zero, as a tensor-map load fills them.
-static __global__ void __launch_bounds__(128) grid_split_operand(const float* __restrict__ vis, int64_t rows, int nbl,
-                                                                 int T, int C, int ntb, unsigned char* __restrict__ out,
-                                                                 float* __restrict__ vinv) {
-  __shared__ float smax[4][32];
+// Builds the split grid operand of a 4-pol complex<float> integration [C][rows][8 floats], one block per (quad,
+// timestep block).  The power of two of each (baseline, pol) brings its largest |component| over the block's 4
+// timesteps and all channels into [2^13, 2^14); vinv holds its inverse (1 for an all-zero one).  hi is the scaled
+// visibility rounded to FP16, lo the remainder rounded to FP16.  Rows and channels past the integration are zero,
+// as a tensor-map load fills them.
+//
+// Bound by HBM: the visibilities read once, the operand (as many bytes) written.  A lane reads 16 bytes, two pols of
+// (timestep lane / 8, baseline (lane / 2) % 4), and writes 64-byte runs of the operand, 8 channels of its 4 rows;
+// the second pass over the tile (after the maxima) finds it in L2: kGrSplitBlocks blocks per SM hold 152 x 2 x
+// 192 KB = 60 MB at 384 channels, and the operand's lines are written evict-first (3 blocks per SM: 0.8 ms).  (4-byte lanes, one channel at a time: 856 us for the 128-antenna integration of
+// 1.42 GB, 510 us now.)
+constexpr int kGrSplitThreads = 512;
+constexpr int kGrSplitBlocks = 2;  // per SM
+static __global__ void __launch_bounds__(kGrSplitThreads, kGrSplitBlocks)
+    grid_split_operand(const float* __restrict__ vis, int64_t rows, int nbl, int T, int C, int ntb,
+                       unsigned char* __restrict__ out, float* __restrict__ vinv) {
+  constexpr int NW = kGrSplitThreads / 32;
+  __shared__ float smax[NW][8][2];
   const int q = blockIdx.x, tb = blockIdx.y, nchunk = (C + kGrChunk - 1) / kGrChunk;
-  const int lane = threadIdx.x & 31, tl = threadIdx.x >> 5;
-  const int t = tb * 4 + tl, b = q * 4 + (lane >> 3);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tl = lane >> 3, bl = (lane >> 1) & 3, half = lane & 1;
+  const int t = tb * 4 + tl, b = q * 4 + bl;
   const bool rv = t < T && b < nbl;
-  const float* src = vis + (static_cast<int64_t>(t) * nbl + b) * 8 + (lane & 7);
-  const int64_t cstride = rows * 8;
-  float m = 0.f;
-  if (rv)
-    for (int c = 0; c < C; ++c) m = fmaxf(m, fabsf(__ldg(src + c * cstride)));
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));  // re and im
-  smax[tl][lane] = m;
+  const float4* src = reinterpret_cast<const float4*>(vis) + (rv ? (static_cast<int64_t>(t) * nbl + b) * 2 + half : 0);
+  const int64_t cstride = rows * 2;
+  auto load = [&](int c) { return rv && c < C ? __ldg(src + c * cstride) : make_float4(0.f, 0.f, 0.f, 0.f); };
+  float m0 = 0.f, m1 = 0.f;  // this lane's two pols
+  for (int i = warp; i < 2 * nchunk; i += NW) {
+    float4 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = load(i * 8 + k);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      m0 = fmaxf(m0, fmaxf(fabsf(v[k].x), fabsf(v[k].y)));
+      m1 = fmaxf(m1, fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
+    }
+  }
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) {  // over the timesteps
+    m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+  if (tl == 0) {
+    smax[warp][lane][0] = m0;
+    smax[warp][lane][1] = m1;
+  }
   __syncthreads();
-  m = fmaxf(fmaxf(smax[0][lane], smax[1][lane]), fmaxf(smax[2][lane], smax[3][lane]));
-  int e = 0;
-  (void)frexpf(m, &e);  // m < 2^e
-  const float scale = m > 0.f ? ldexpf(1.f, 14 - e) : 1.f;
-  if (tl == 0 && !(lane & 1)) vinv[(static_cast<int64_t>(q) * ntb + tb) * 16 + (lane >> 1)] = 1.f / scale;
-  const int mrow = (lane >> 3) * 32 + tl * 8 + (lane & 7);  // TMEM lane: baseline, timestep, pol, re/im
-  for (int chunk = 0; chunk < nchunk; ++chunk) {
-    unsigned char* dst = out + ((static_cast<int64_t>(q) * ntb + tb) * nchunk + chunk) * kGrOpBytes;
+  float scale[2];
 #pragma unroll
-    for (int kh = 0; kh < 2; ++kh) {
-      uint32_t hw[4], lw[4];
+  for (int p = 0; p < 2; ++p) {
+    float m = 0.f;
+    for (int w = 0; w < NW; ++w) m = fmaxf(m, smax[w][lane & 7][p]);
+    int e = 0;
+    (void)frexpf(m, &e);  // m < 2^e
+    scale[p] = m > 0.f ? ldexpf(1.f, 14 - e) : 1.f;
+    if (warp == 0 && tl == 0) vinv[(static_cast<int64_t>(q) * ntb + tb) * 16 + bl * 4 + half * 2 + p] = 1.f / scale[p];
+  }
+  const int mrow = bl * 32 + tl * 8 + half * 4;  // first of this lane's 4 rows: baseline, timestep, pol, re/im
+  for (int i = warp; i < 2 * nchunk; i += NW) {
+    float4 v[8];
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        float x[2];
+    for (int k = 0; k < 8; ++k) v[k] = load(i * 8 + k);
+    unsigned char* dst = out + ((static_cast<int64_t>(q) * ntb + tb) * nchunk + (i >> 1)) * kGrOpBytes +
+                         grid_f16_offset(mrow, (i & 1) * 8);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int c = chunk * kGrChunk + kh * 8 + j + i;
-          x[i] = (rv && c < C) ? __ldg(src + c * cstride) * scale : 0.f;
+    for (int r0 = 0; r0 < 4; r0 += 2) {  // rows r0 and r0 + 1: (re, im) of one pol
+      uint32_t hw[8], lw[8];
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          const float x0 = (r0 == 0 ? (r == 0 ? v[k].x : v[k].y) : (r == 0 ? v[k].z : v[k].w)) * scale[r0 >> 1];
+          const float x1 = (r0 == 0 ? (r == 0 ? v[k + 1].x : v[k + 1].y) : (r == 0 ? v[k + 1].z : v[k + 1].w)) * scale[r0 >> 1];
+          const __half2 h = __floats2half2_rn(x0, x1);
+          const __half2 l = __floats2half2_rn(x0 - __low2float(h), x1 - __high2float(h));
+          hw[r * 4 + (k >> 1)] = *reinterpret_cast<const uint32_t*>(&h);
+          lw[r * 4 + (k >> 1)] = *reinterpret_cast<const uint32_t*>(&l);
         }
-        const __half2 h = __floats2half2_rn(x[0], x[1]);
-        const __half2 l = __floats2half2_rn(x[0] - __low2float(h), x[1] - __high2float(h));
-        hw[j >> 1] = *reinterpret_cast<const uint32_t*>(&h);
-        lw[j >> 1] = *reinterpret_cast<const uint32_t*>(&l);
+#pragma unroll
+      for (int hl = 0; hl < 2; ++hl) {  // 32 bytes, 32-byte aligned
+        const uint32_t(&w)[8] = hl == 0 ? hw : lw;
+        asm volatile("st.global.L2::evict_first.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + hl * kGrAHalf + r0 * 16), "r"(w[0]),
+                     "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
       }
-      const int off = grid_f16_offset(mrow, kh * 8);
-      *reinterpret_cast<uint4*>(dst + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-      *reinterpret_cast<uint4*>(dst + kGrAHalf + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
     }
   }
 }

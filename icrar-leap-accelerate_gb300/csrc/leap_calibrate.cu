@@ -120,7 +120,7 @@ int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const doubl
       if (ctx->capturing) return fail(ctx, LEAP_ERR_INTERNAL, "grid operand missing while recording a graph");
       LEAP_CUDA(in.op.ensure(static_cast<size_t>(op_bytes + grid_scale_bytes(nbl, T))), "alloc grid operand");
       const dim3 og((nbl + 3) / 4, (T + 3) / 4);
-      grid_split_operand<<<og, 128, 0, s>>>(in.vis.as<float>(), in.rows, nbl, T, C, (T + 3) / 4,
+      grid_split_operand<<<og, kGrSplitThreads, 0, s>>>(in.vis.as<float>(), in.rows, nbl, T, C, (T + 3) / 4,
                                             in.op.as<unsigned char>(),
                                             reinterpret_cast<float*>(in.op.as<unsigned char>() + op_bytes));
       LEAP_CUDA(cudaGetLastError(), "grid operand launch");
