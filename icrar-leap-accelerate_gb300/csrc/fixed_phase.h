@@ -19,7 +19,7 @@
 //
 // Numbers in [-1, 1] are 60-bit fixed point in two limbs of radix 2^30: x = (h 2^30 + l) 2^-60, l in
 // [0, 2^30).  Products of limbs go to 64-bit sums (IMAD.WIDE: 32 lanes per clock and SM measured, where
-// FP64 FMAs run at 2); the product of the two low limbs is dropped, its mean added back.  60 bits, not
+// FP64 FMAs run at 2); the product of the two low limbs is dropped.  60 bits, not
 // fewer, because the rounding of the channel step's phasor adds up over the channels of a block: with
 // 56 bits the phasors were up to 50 units of 2^-56 off after 32 channels.
 #pragma once
@@ -86,17 +86,43 @@ LEAP_HD int32_t fx_clz(uint32_t x) {
 #endif
 }
 
-// acc += a * b.  On the device as a carry pair, which the assembler fuses to one IMAD.WIDE: from mad.wide it
+// a * b + c.  On the device as a carry pair, which the assembler fuses to one IMAD.WIDE: from mad.wide it
 // makes a product and a two-instruction addition where a sum gets several products in a row, and from the
-// plain expression 64-bit products of limbs that were cut out of 64-bit numbers.
-LEAP_HD void fx_mad(int64_t& acc, int32_t a, int32_t b) {
+// plain expression 64-bit products of limbs that were cut out of 64-bit numbers.  (A constant c keeps the pair
+// from being fused: a sum starts with fx_mul.)
+LEAP_HD int64_t fx_mad(int32_t a, int32_t b, int64_t c) {
 #ifdef __CUDA_ARCH__
-  asm("{\n\t.reg .u32 l, h;\n\tmov.b64 {l, h}, %0;\n\tmad.lo.cc.s32 l, %1, %2, l;\n\tmadc.hi.s32 h, %1, %2, h;\n\t"
+  int64_t r;
+  asm("{\n\t.reg .u32 l, h;\n\tmov.b64 {l, h}, %3;\n\tmad.lo.cc.s32 l, %1, %2, l;\n\tmadc.hi.s32 h, %1, %2, h;\n\t"
       "mov.b64 %0, {l, h};\n\t}"
-      : "+l"(acc)
-      : "r"(a), "r"(b));
+      : "=l"(r)
+      : "r"(a), "r"(b), "l"(c));
+  return r;
 #else
-  acc += static_cast<int64_t>(a) * b;
+  return c + static_cast<int64_t>(a) * b;
+#endif
+}
+
+LEAP_HD void fx_mad(int64_t& acc, int32_t a, int32_t b) { acc = fx_mad(a, b, acc); }
+
+LEAP_HD int64_t fx_mul(int32_t a, int32_t b) {
+#ifdef __CUDA_ARCH__
+  int64_t r;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+#else
+  return static_cast<int64_t>(a) * b;
+#endif
+}
+
+// (a * b >> 32) + c
+LEAP_HD int32_t fx_mad_hi(int32_t a, int32_t b, int32_t c) {
+#ifdef __CUDA_ARCH__
+  int32_t r;
+  asm("mad.hi.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+  return r;
+#else
+  return static_cast<int32_t>((static_cast<int64_t>(a) * b) >> 32) + c;
 #endif
 }
 
@@ -105,15 +131,10 @@ LEAP_HD FxLimbs fx_limbs(int64_t re, int64_t im) {
                  static_cast<int32_t>(im >> 30), static_cast<int32_t>(static_cast<uint32_t>(im) & (kFxLimb - 1))};
 }
 
-// x * y as 60-bit integers.  The constant of the imaginary part's sum also puts back the mean of the
-// dropped low products (which cancel in the real part).
-LEAP_HD void fx_product(const FxLimbs& x, const FxLimbs& y, int64_t& re, int64_t& im) {
-  const int32_t nih = -x.ih, nil = -x.il;
-    int64_t hr = 0, hi = 0, mr = int64_t(1) << 29, mi = int64_t(1) << 30;
-  fx_mad(hr, x.rh, y.rh);
-  fx_mad(hi, x.rh, y.ih);
-  fx_mad(mr, x.rh, y.rl);
-  fx_mad(mi, x.rh, y.il);
+// x * y as 60-bit integers, rounded down.  (nih, nil): the limbs of -im(x), not the negated ones: of a plainly
+// negated operand the assembler makes an IMAD and an IMAD.HI instead of an IMAD.WIDE.
+LEAP_HD void fx_product(const FxLimbs& x, int32_t nih, int32_t nil, const FxLimbs& y, int64_t& re, int64_t& im) {
+  int64_t hr = fx_mul(x.rh, y.rh), hi = fx_mul(x.rh, y.ih), mr = fx_mul(x.rh, y.rl), mi = fx_mul(x.rh, y.il);
   fx_mad(hr, nih, y.ih);
   fx_mad(hi, x.ih, y.rh);
   fx_mad(mr, x.rl, y.rh);
@@ -128,7 +149,7 @@ LEAP_HD void fx_product(const FxLimbs& x, const FxLimbs& y, int64_t& re, int64_t
 
 LEAP_HD FxLimbs fx_cmul(const FxLimbs& x, const FxLimbs& y) {
   int64_t re, im;
-  fx_product(x, y, re, im);
+  fx_product(x, -x.ih, -x.il, y, re, im);
   return fx_limbs(re, im);
 }
 
@@ -168,11 +189,9 @@ LEAP_HD uint64_t fx_bits(double x) {
 // lambda_c).  At most (512 + kFxMaxRho / 2) LSB: below 2^30.
 LEAP_HD int32_t fx_residual(const FxPhase& ph, int32_t rho) {
   const int32_t hi = static_cast<int32_t>(ph.v >> 32);
-  int64_t term = 0;
-  fx_mad(term, hi, rho);
   // The low 32 - kFxFrac bits of the phase and kFxFrac bits of its fraction.
   const uint32_t x = (static_cast<uint32_t>(ph.v) << kFxFrac) | (ph.vf >> (32 - kFxFrac));
-  const uint32_t y = x + static_cast<uint32_t>(term >> 32);
+  const uint32_t y = static_cast<uint32_t>(fx_mad_hi(hi, rho, static_cast<int32_t>(x)));
   const int lz = fx_clz(static_cast<uint32_t>(hi) ^ ph.sign) - 1;  // 0 .. 31: the argument is below 2^(E - lz)
   const int32_t mask = -(1 << (10 + kFxFrac)) >> lz;               // its last place is 2^(10 - lz) LSBs
   const uint32_t half = (1u << (9 + kFxFrac)) >> lz;
@@ -217,9 +236,9 @@ LEAP_HD uint64_t fx_turns(const FxPhase& ph) {
   return neg ? ~t + 1 : t;
 }
 
-// One channel on: the phase, its residual, and the step's small turn in units of 2^-62 rad, below 2^31 as
-// residuals are below 2^30 (an LSB is 2^(E-1) of these units, E - 1 <= kFxFrac).
-LEAP_HD int32_t fx_advance(FxPhase& ph, int32_t rho) {
+// One channel on: the phase, its residual, and the step's small turn d in units of 2^-62 rad, below 2^31 as
+// residuals are below 2^30 (an LSB is 2^(E-1) of these units, E - 1 <= kFxFrac); nd = -d to a unit.
+LEAP_HD void fx_advance(FxPhase& ph, int32_t rho, int32_t& d, int32_t& nd) {
 #ifdef __CUDA_ARCH__
   uint32_t lo = static_cast<uint32_t>(ph.v), hi = static_cast<uint32_t>(ph.v >> 32);
   asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
@@ -233,27 +252,21 @@ LEAP_HD int32_t fx_advance(FxPhase& ph, int32_t rho) {
   ph.vf = static_cast<uint32_t>(s);
 #endif
   const int32_t e = fx_residual(ph, rho);
-  const int32_t d = e - ph.e;
+  d = (e - ph.e) >> (kFxFrac + 1 - ph.E);
+  nd = (ph.e - e) >> (kFxFrac + 1 - ph.E);
   ph.e = e;
-  return d >> (kFxFrac + 1 - ph.E);
 }
 static_assert(kFxMaxExp <= kFxFrac + 1, "the shift of a residual's difference");
 
-// w turned by the small angle d (2^-62 rad): its low limbs change, by less than 2^30.
-LEAP_HD FxLimbs fx_turned(const FxLimbs& w, int32_t d) {
-  int64_t re = (static_cast<int64_t>(w.rl) << 32) + (int64_t(1) << 31);
-  int64_t im = (static_cast<int64_t>(w.il) << 32) + (int64_t(1) << 31);
-  fx_mad(re, -d, w.ih);
-  fx_mad(im, d, w.rh);
-  FxLimbs r = w;
-  r.rl = static_cast<int32_t>(re >> 32);
-  r.il = static_cast<int32_t>(im >> 32);
-  return r;
-}
-
-// The phasor z = (re, im) of one channel times the step w, turned by d.
-LEAP_HD void fx_step(int64_t& re, int64_t& im, const FxLimbs& w, int32_t d) {
-  fx_product(fx_limbs(re, im), fx_turned(w, d), re, im);
+// The phasor z = (re, im) of one channel times the step w turned by the small angle d (2^-62 rad, nd = -d), which
+// changes the low limbs of w by less than 2^30.
+LEAP_HD void fx_step(int64_t& re, int64_t& im, const FxLimbs& w, int32_t d, int32_t nd) {
+  FxLimbs turned = w;
+  turned.rl = fx_mad_hi(nd, w.ih, w.rl);
+  turned.il = fx_mad_hi(d, w.rh, w.il);
+  const int64_t n = -im;
+  fx_product(fx_limbs(re, im), static_cast<int32_t>(n >> 30), static_cast<int32_t>(static_cast<uint32_t>(n) & (kFxLimb - 1)),
+             turned, re, im);
 }
 
 }  // namespace leapgb

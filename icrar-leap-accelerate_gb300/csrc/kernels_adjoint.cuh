@@ -436,14 +436,13 @@ __global__ void __launch_bounds__(128, 3) adjoint_vis_fixed(const AdjointFixedAr
     ray.seed(__ldg(f.rho + c0), f.tab);
     constexpr float kUnit = FxSumFloat<1>::kUnit;
     const float lx = __int_as_float(g.y), ly = __int_as_float(g.w), hx = g.x * kUnit, hy = g.z * kUnit;
-    const int32_t ngx = -g.x;
 #pragma unroll
     for (int k = 0; k < kVisChannels; ++k) {
       const typename FxSumFloat<1>::Phasor z = FxSumFloat<1>::phasor(ray.zr, ray.zi);
       fx_mad(hr[k], g.x, z.rh);  // re: g.x z.r + g.y z.i; im: g.y z.r - g.x z.i
       fx_mad(hi[k], g.z, z.rh);
       fx_mad(hr[k], g.z, z.ih);
-      fx_mad(hi[k], ngx, z.ih);
+      fx_mad(hi[k], g.x, z.nih);
       mr[k] = fmaf(lx, z.rhf, fmaf(hx, z.rlf, mr[k]));
       mi[k] = fmaf(ly, z.rhf, fmaf(hy, z.rlf, mi[k]));
       mr[k] = fmaf(ly, z.ihf, fmaf(hy, z.ilf, mr[k]));

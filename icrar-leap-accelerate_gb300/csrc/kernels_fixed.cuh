@@ -154,13 +154,19 @@ struct FxSumInt {
     for (int p = 0; p < P; ++p) hh[p][0] = hh[p][1] = mid[p][0] = mid[p][1] = 0;
   }
   struct Phasor {
-    int32_t rh, rl, ih, il;
+    int32_t rh, rl, ih, il, nih, nil;  // (nih, nil): the negated imaginary part
   };
   // 56 bits of a 60-bit phasor, rounded, in limbs of radix 2^27.
+  static __device__ __forceinline__ void limbs(int64_t x, int32_t& h, int32_t& l) {
+    h = static_cast<int32_t>(x >> 31);
+    l = static_cast<int32_t>((static_cast<uint32_t>(x) >> 4) & 0x7FFFFFFu);
+  }
   static __device__ __forceinline__ Phasor phasor(int64_t zr, int64_t zi) {
-    const int64_t fr = zr + 8, fi = zi + 8;
-    return Phasor{static_cast<int32_t>(fr >> 31), static_cast<int32_t>((static_cast<uint32_t>(fr) >> 4) & 0x7FFFFFFu),
-                  static_cast<int32_t>(fi >> 31), static_cast<int32_t>((static_cast<uint32_t>(fi) >> 4) & 0x7FFFFFFu)};
+    Phasor z;
+    limbs(zr + 8, z.rh, z.rl);
+    limbs(zi + 8, z.ih, z.il);
+    limbs(8 - zi, z.nih, z.nil);
+    return z;
   }
   struct Vis {
     int4 v[P];  // (re h, re l, im h, im l)
@@ -184,7 +190,7 @@ struct FxSumInt {
     return r;
   }
   __device__ __forceinline__ void add(const Vis& x, const Phasor& z) {
-    const int32_t nih = -z.ih, nil = -z.il;
+    const int32_t nih = z.nih, nil = z.nil;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
       const int4 v = x.v[p];
@@ -229,13 +235,14 @@ struct FxSumFloat {
     }
   }
   struct Phasor {
-    int32_t rh, ih;
+    int32_t rh, ih, nih;  // nih = -ih
     float rhf, rlf, ihf, ilf;
   };
   static __device__ __forceinline__ Phasor phasor(int64_t zr, int64_t zi) {
     Phasor z;
     z.rh = static_cast<int32_t>((zr + (int64_t(1) << 31)) >> 32);
     z.ih = static_cast<int32_t>((zi + (int64_t(1) << 31)) >> 32);
+    z.nih = static_cast<int32_t>(((int64_t(1) << 31) - 1 - zi) >> 32);  // as such: see fx_product
     z.rlf = static_cast<float>(static_cast<int32_t>(zr));
     z.ilf = static_cast<float>(static_cast<int32_t>(zi));
     z.rhf = static_cast<float>(z.rh);
@@ -292,12 +299,11 @@ struct FxSumFloat {
     return r;
   }
   __device__ __forceinline__ void add(const Vis& x, const Phasor& z) {
-    const int32_t nih = -z.ih;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
       fx_mad(hh[p][0], x.h[p][0], z.rh);
       fx_mad(hh[p][1], x.h[p][0], z.ih);
-      fx_mad(hh[p][0], x.h[p][1], nih);
+      fx_mad(hh[p][0], x.h[p][1], z.nih);
       fx_mad(hh[p][1], x.h[p][1], z.rh);
       ra[p] = fmaf(x.l[p][0], z.rhf, fmaf(x.hf[p][0], z.rlf, ra[p]));
       ra[p] = fmaf(x.l[p][1], -z.ihf, fmaf(x.hf[p][1], -z.ilf, ra[p]));
@@ -348,7 +354,11 @@ struct FxRay {
     zr = fits ? (static_cast<int64_t>(z.rh) << 30) + z.rl : 0;
     zi = fits ? (static_cast<int64_t>(z.ih) << 30) + z.il : 0;
   }
-  __device__ __forceinline__ void next(int32_t rho) { fx_step(zr, zi, w, fx_advance(ph, rho)); }
+  __device__ __forceinline__ void next(int32_t rho) {
+    int32_t d, nd;
+    fx_advance(ph, rho, d, nd);
+    fx_step(zr, zi, w, d, nd);
+  }
 };
 
 // sf = -2 pi (w_rot - w) of a row, without fused operations, as the reference forms it.

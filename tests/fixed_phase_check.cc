@@ -27,7 +27,11 @@ extern "C" int fx_check(double sf, double f0, double df, int channels, const dou
     }
     zr[c - c0] = re;
     zi[c - c0] = im;
-    if (c + 1 < channels) fx_step(re, im, w, fx_advance(ph, rho[c + 1]));
+    if (c + 1 < channels) {
+      int32_t d, nd;
+      fx_advance(ph, rho[c + 1], d, nd);
+      fx_step(re, im, w, d, nd);
+    }
   }
   return 0;
 }
