@@ -104,7 +104,14 @@ constexpr int kGrEOffset = kGrOpBytes;
 constexpr int kGrRecWords = 16;                          // per (direction, timestep) record: 4 16-byte rows
 constexpr int kGrCodeWord = kGrTaps + 3;                 // record: W + 1 weights, cr, sr, then the load code
 constexpr int kGrRecDirs = 16;                           // directions whose records a warp holds at a time
-constexpr int kGrRecBytes = kGrEpiWarps * 4 * kGrRecDirs * kGrRecWords * 4;  // [warps][4 t][16 dirs][12]
+// Records in shared memory, [warps][4 t][16 dirs]: a timestep's records are 16 bytes past a multiple of 128, so that
+// the 4 timesteps of a warp's lanes read one row of a direction from different banks, and the rows of a record are
+// exchanged with its direction's bits 1 and 2, so that the 8 lanes of a timestep write one row of theirs without
+// conflicts either.  (Without both the records took 7 to 9 of a tile's 17 thousand cycles of shared memory, beside 4
+// of the MMAs' operands and 2.7 of the copies: the bound of the kernel.  128 antennas: REC0 -> REC1 ms a call.)
+constexpr int kGrRecStep = kGrRecDirs * kGrRecWords + 4;  // words per timestep
+constexpr int kGrRecBytes = kGrEpiWarps * 4 * kGrRecStep * 4;
+__host__ __device__ constexpr int grid_rec_row(int j, int i) { return j * kGrRecWords + ((i ^ ((j >> 1) & 3)) << 2); }
 constexpr uint32_t kGrRegion = 128;                      // TMEM columns per region
 constexpr uint32_t kGrIS = 2 * kGrRegion, kGrAC = 3 * kGrRegion;
 constexpr int kGrWide = 1 << 16;                         // record flag: the 4 timesteps need separate loads
@@ -437,31 +444,27 @@ __device__ __forceinline__ void grid_weights(float f, bool shifted, const float 
   w[W] = shifted ? h[W - 1] : 0.f;
 }
 
-// Two directions' stencils from TMEM: a 16-, a 4- and a 2-column load each (the W + 1 = 11
-// taps, re and im interleaved) at columns c0 and c1 of this warp's lanes, and one wait for both.
+// A stencil's taps from TMEM: a 16-, a 4- and a 2-column load (the W + 1 = 11 taps, re and im interleaved) at
+// column c of this warp's lanes.  The registers hold them only after grid_load_wait of the same array.
 constexpr int kGrLoadRegs = 2 * kGrLoadCols;
 static_assert(kGrLoadRegs == 22, "22 columns per stencil: x16 + x4 + x2 loads");
-__device__ __forceinline__ void grid_load_pair(uint32_t tbase, uint32_t c0, uint32_t c1,
-                                               uint32_t (&v)[2][kGrLoadRegs]) {
-  // All loads and the wait in one statement: the results are defined only after the wait.
+__device__ __forceinline__ void grid_load_start(uint32_t a0, uint32_t (&v)[kGrLoadRegs]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%44];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16,%17,%18,%19}, [%45];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%20,%21}, [%46];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,%35,%36,%37}, [%47];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%38,%39,%40,%41}, [%48];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%42,%43}, [%49];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(v[0][0]), "=r"(v[0][1]), "=r"(v[0][2]), "=r"(v[0][3]), "=r"(v[0][4]), "=r"(v[0][5]), "=r"(v[0][6]),
-        "=r"(v[0][7]), "=r"(v[0][8]), "=r"(v[0][9]), "=r"(v[0][10]), "=r"(v[0][11]), "=r"(v[0][12]), "=r"(v[0][13]),
-        "=r"(v[0][14]), "=r"(v[0][15]), "=r"(v[0][16]), "=r"(v[0][17]), "=r"(v[0][18]), "=r"(v[0][19]),
-        "=r"(v[0][20]), "=r"(v[0][21]),
-        "=r"(v[1][0]), "=r"(v[1][1]), "=r"(v[1][2]), "=r"(v[1][3]), "=r"(v[1][4]), "=r"(v[1][5]), "=r"(v[1][6]),
-        "=r"(v[1][7]), "=r"(v[1][8]), "=r"(v[1][9]), "=r"(v[1][10]), "=r"(v[1][11]), "=r"(v[1][12]), "=r"(v[1][13]),
-        "=r"(v[1][14]), "=r"(v[1][15]), "=r"(v[1][16]), "=r"(v[1][17]), "=r"(v[1][18]), "=r"(v[1][19]),
-        "=r"(v[1][20]), "=r"(v[1][21])
-      : "r"(tbase + c0), "r"(tbase + c0 + 16u), "r"(tbase + c0 + 20u), "r"(tbase + c1), "r"(tbase + c1 + 16u),
-        "r"(tbase + c1 + 20u));
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%22];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16,%17,%18,%19}, [%23];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%20,%21}, [%24];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21])
+      : "r"(a0), "r"(a0 + 16u), "r"(a0 + 20u));
+}
+
+// Waits for every load of this warp so far; v passes through, so that nothing reads it before.
+__device__ __forceinline__ void grid_load_wait(uint32_t (&v)[kGrLoadRegs]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
+                 "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]));
 }
 
 // One stencil from TMEM (a 16-, a 4- and a 2-column load) and its wait.
@@ -482,12 +485,12 @@ __device__ __forceinline__ void grid_load_one(uint32_t a0, uint32_t (&v)[kGrLoad
 // partner lane (the other component of the same visibility); returns this lane's
 // component of the rotated sum.  sgn is -1 on the real lane (comp 0), +1 on the imaginary.
 template <int W>
-__device__ __forceinline__ float grid_tap_combine(const uint32_t (&v)[kGrLoadRegs], const float* rec, float sgn) {
+__device__ __forceinline__ float grid_tap_combine(const uint32_t (&v)[kGrLoadRegs], const float* rec_t, int j, float sgn) {
   static_assert(W + 1 == kGrLoadCols && kGrRecWords == 16, "record layout: W + 1 weights, then cr, sr, code");
   float r[16];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float4 q = reinterpret_cast<const float4*>(rec)[i];
+    const float4 q = *reinterpret_cast<const float4*>(rec_t + grid_rec_row(j, i));
     r[4 * i] = q.x;
     r[4 * i + 1] = q.y;
     r[4 * i + 2] = q.z;
@@ -517,18 +520,18 @@ __device__ __forceinline__ float grid_tap_combine(const uint32_t (&v)[kGrLoadReg
 }
 
 // A direction whose 4 timesteps need separate grid windows: one load per timestep
-// (rare; kept out of line so that the common path stays small).  rec_dir is the
-// direction's record at timestep 0; timestep t's is t * kGrRecDirs records further.
+// (rare; kept out of line so that the common path stays small).  rec holds the warp's
+// records, j is the direction.
 template <int W>
-__device__ __noinline__ float grid_wide_sum(const float* rec_dir, uint32_t tbase, float sgn, int tl, int pp) {
+__device__ __noinline__ float grid_wide_sum(const float* rec, int j, uint32_t tbase, float sgn, int tl, int pp) {
   float acc = 0.f;
   for (int tt = 0; tt < 4; ++tt) {
-    const float* r = rec_dir + tt * kGrRecDirs * kGrRecWords;
-    const int ct = __float_as_int(r[kGrCodeWord]);
+    const float* r = rec + tt * kGrRecStep;
+    const int ct = __float_as_int(r[grid_rec_row(j, kGrCodeWord / 4) + kGrCodeWord % 4]);
     if ((ct & 0xFFFF) == 0xFFFF || ((ct >> 8) & 255) != pp) continue;  // same in every lane
     uint32_t v[kGrLoadRegs];
     grid_load_one(tbase + 2u * static_cast<uint32_t>(ct & 255), v);
-    const float g = grid_tap_combine<W>(v, r, sgn);
+    const float g = grid_tap_combine<W>(v, r, j, sgn);
     if (tl == tt) acc += g;
   }
   return acc;
@@ -543,7 +546,7 @@ __device__ __noinline__ float grid_wide_sum(const float* rec_dir, uint32_t tbase
 template <int W>
 __device__ __forceinline__ void grid_record(const GridParams& p, const float (&x)[6], const float2* tab, int d,
                                             bool dv, bool rval, int n, int c0, int lbase, int r0, int npass,
-                                            float* dst) {
+                                            float* rec_t, int j) {
   float ka[6], kb[6];
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
@@ -580,11 +583,11 @@ __device__ __forceinline__ void grid_record(const GridParams& p, const float (&x
   float cr, sr;
   twiddle_turns(pa + static_cast<uint32_t>(c0) * pb, tab, cr, sr);
   static_assert(W == 10 && kGrCodeWord == 13 && kGrRecWords == 16, "record layout");
-  float4* my = reinterpret_cast<float4*>(dst);
-  my[0] = make_float4(wt[0], wt[1], wt[2], wt[3]);
-  my[1] = make_float4(wt[4], wt[5], wt[6], wt[7]);
-  my[2] = make_float4(wt[8], wt[9], wt[10], cr);
-  my[3] = make_float4(sr, __int_as_float(code), 0.f, 0.f);
+  auto row = [&](int i) { return reinterpret_cast<float4*>(rec_t + grid_rec_row(j, i)); };
+  *row(0) = make_float4(wt[0], wt[1], wt[2], wt[3]);
+  *row(1) = make_float4(wt[4], wt[5], wt[6], wt[7]);
+  *row(2) = make_float4(wt[8], wt[9], wt[10], cr);
+  *row(3) = make_float4(sr, __int_as_float(code), 0.f, 0.f);
 }
 
 // Sum of TMEM regions into the first one, for this warp's 32 lanes and columns
@@ -693,6 +696,16 @@ __device__ __forceinline__ void grid_flush(const float (&acc)[kGrWarpDirs / kGrB
   }
 }
 
+// One lane of a converged warp, the same in every call.
+__device__ __forceinline__ bool grid_elect() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
+// Lane 0's value, which the compiler then knows to be the same in the whole warp.
+__device__ __forceinline__ int grid_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 template <int W>
 __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const GridParams p) {
   extern __shared__ __align__(128) unsigned char grid_smem[];
@@ -781,70 +794,79 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      uint32_t ctr = 0, blk = 0, mids = 0;
-      bool ok = true, issued = false;
-      for (int sl = blockIdx.x; ok; sl += gridDim.x) {
-        const int u = sl < p.nslots ? __ldg(p.order + sl) : -1;
-        if (u < 0) break;
-        const GridUnit g = grid_unit(p, u);
-        const GridItem& I = p.items[g.item];
-        const GridWindow w = p.win[u];
-        const uint32_t idesc = grid_idesc_f16(128, 2 * w.jw);
-        const uint64_t adesc0 = tc_smem_desc(ve, kTcLbo, kTcSbo);
-        const uint64_t edesc0 = tc_smem_desc(ve + kGrEOffset, kTcLbo, kTcSbo);
-        for (int tb = 0; tb < g.ntb && ok; ++tb)
-          for (int ps = 0; ps < w.npass && ok; ++ps, ++blk) {
-            const uint32_t b = blk & 1;
-            if ((blk >= 2 && !grid_wait(&rs_free[b], ((blk >> 1) - 1) & 1, abort_flag)) ||
-                (blk >= 1 && !grid_wait(ac_free, (blk - 1) & 1, abort_flag))) {
-              grid_fail(p, abort_flag);
+    // The whole warp walks the units, so that descriptors are warp-uniform (held in uniform registers, where
+    // tcgen05.mma reads them), and one elected lane issues a segment's 12 MMAs from straight-line code.
+    const bool lead = grid_elect();
+    uint32_t ctr = 0, blk = 0, mids = 0;
+    bool ok = true, issued = false;
+    const uint64_t adesc0 = tc_smem_desc(ve, kTcLbo, kTcSbo);
+    const uint64_t edesc0 = tc_smem_desc(ve + kGrEOffset, kTcLbo, kTcSbo);
+    for (int sl = blockIdx.x; ok; sl += gridDim.x) {
+      const int u = grid_uniform(sl < p.nslots ? __ldg(p.order + sl) : -1);
+      if (u < 0) break;
+      const GridUnit g = grid_unit(p, u);
+      const int ntb = grid_uniform(g.ntb), nchunk = grid_uniform(p.items[g.item].nchunk);
+      const int jw = grid_uniform(p.win[u].jw), npass = grid_uniform(p.win[u].npass);
+      const uint32_t idesc = grid_idesc_f16(128, 2 * jw);
+      const uint64_t elo = static_cast<uint64_t>(2 * jw * 2);  // E lo after E hi, in descriptor units of 16 bytes
+      for (int tb = 0; tb < ntb && ok; ++tb)
+        for (int ps = 0; ps < npass && ok; ++ps, ++blk) {
+          const uint32_t b = blk & 1;
+          if ((blk >= 2 && !grid_wait(&rs_free[b], ((blk >> 1) - 1) & 1, abort_flag)) ||
+              (blk >= 1 && !grid_wait(ac_free, (blk - 1) & 1, abort_flag))) {
+            if (lead) grid_fail(p, abort_flag);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t rs = tmem + b * kGrRegion;
+          for (int q0 = 0; q0 < nchunk && ok; q0 += kGrMacro, ++ctr) {
+            const int m = ctr % kGrMacroStages;
+            const int nq = min(kGrMacro, nchunk - q0);
+            if (!grid_wait(&vfull[m], (ctr / kGrMacroStages) & 1, abort_flag)) {
+              if (lead) grid_fail(p, abort_flag);
               ok = false;
               break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t rs = tmem + b * kGrRegion;
-            for (int q0 = 0; q0 < I.nchunk && ok; q0 += kGrMacro, ++ctr) {
-              const int m = ctr % kGrMacroStages;
-              const int nq = min(kGrMacro, I.nchunk - q0);
-              if (!grid_wait(&vfull[m], (ctr / kGrMacroStages) & 1, abort_flag)) {
-                grid_fail(p, abort_flag);
-                ok = false;
-                break;
-              }
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              // A round is one segment.  Its correction MMAs go first: they give the fold of the
-              // previous segment time to finish before the hi*hi MMAs restart IS.
-              const int seg = q0 / kGrSegChunks;
-              // Descriptors of stage i: A hi/lo at +0 / +kGrAHalf, E hi/lo at +0 / +2*jw*32 from their
-              // bases (address field >> 4).
-              const uint64_t so0 = static_cast<uint64_t>(m * kGrMacro * (kGrStageBytes >> 4));
-              const uint64_t sst = static_cast<uint64_t>(kGrStageBytes >> 4);
-              for (int i = 0; i < nq; ++i) {
-                const uint64_t ah = adesc0 + so0 + i * sst, bh = edesc0 + so0 + i * sst;
-                const uint64_t al = ah + (kGrAHalf >> 4), bl = bh + static_cast<uint64_t>(2 * w.jw * 2);
-                grid_mma_corrections(tmem + kGrAC, ah, al, bh, bl, idesc, q0 + i > 0 ? 1u : 0u);
-              }
-              issued = true;
-              if (seg >= 2 && !grid_wait(is_empty, (mids - 1) & 1, abort_flag)) {
-                grid_fail(p, abort_flag);
-                ok = false;
-              } else {
-                const uint32_t dst = seg == 0 ? rs : tmem + kGrIS;
-                for (int i = 0; i < nq; ++i)
-                  grid_mma_hihi(dst, adesc0 + so0 + i * sst, edesc0 + so0 + i * sst, idesc, i > 0 ? 1u : 0u);
-                if (seg >= 1 && q0 + nq < I.nchunk) ++mids;  // a middle segment, folded
-              }
-              if (issued) tc_commit(&sdone[m]);
+            // A round is one segment.  Its correction MMAs go first: they give the fold of the
+            // previous segment time to finish before the hi*hi MMAs restart IS.
+            const int seg = q0 / kGrSegChunks;
+            // Descriptors of stage i: A hi/lo at +0 / +kGrAHalf, E hi/lo at +0 / +2*jw*32 from their
+            // bases (address field >> 4).
+            constexpr uint64_t sst = static_cast<uint64_t>(kGrStageBytes >> 4);
+            const uint64_t ad = adesc0 + m * (kGrMacro * sst), ed = edesc0 + m * (kGrMacro * sst);
+            if (lead) {
+#pragma unroll
+              for (int i = 0; i < kGrMacro; ++i)
+                if (i < nq)
+                  grid_mma_corrections(tmem + kGrAC, ad + i * sst, ad + i * sst + (kGrAHalf >> 4), ed + i * sst,
+                                       ed + i * sst + elo, idesc, q0 + i > 0 ? 1u : 0u);
             }
+            issued = true;
+            if (seg >= 2 && !grid_wait(is_empty, (mids - 1) & 1, abort_flag)) {
+              if (lead) grid_fail(p, abort_flag);
+              ok = false;
+            } else {
+              const uint32_t dst = seg == 0 ? rs : tmem + kGrIS;
+              if (lead) {
+#pragma unroll
+                for (int i = 0; i < kGrMacro; ++i)
+                  if (i < nq) grid_mma_hihi(dst, ad + i * sst, ed + i * sst, idesc, i > 0 ? 1u : 0u);
+              }
+              if (seg >= 1 && q0 + nq < nchunk) ++mids;  // a middle segment, folded
+            }
+            if (lead) tc_commit(&sdone[m]);
+            __syncwarp();
           }
-      }
-      // No MMA of this block may be in flight when its TMEM is freed.
-      if (issued) {
-        const uint32_t j = ctr - 1;
-        if (!mbar_wait_bounded(&sdone[j % kGrMacroStages], (j / kGrMacroStages) & 1)) atomicOr(p.err, kDevErrTimeout);
-      }
+        }
     }
+    // No MMA of this block may be in flight when its TMEM is freed.
+    if (issued && lead) {
+      const uint32_t j = ctr - 1;
+      if (!mbar_wait_bounded(&sdone[j % kGrMacroStages], (j / kGrMacroStages) & 1)) atomicOr(p.err, kDevErrTimeout);
+    }
+    __syncwarp();
   } else if (warp < 6) {
     // ---------------- fold warps: segments and corrections into the running sums ----------------
     const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
@@ -902,10 +924,9 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
     const int quarter = warp & 3;  // TMEM lanes 32*quarter .. (hardware rule: warp id mod 4)
     const int tl = lane >> 3, ps = lane & 7, comp = lane & 1;
     const float sgn = comp ? 1.f : -1.f;
-    // Records of kGrRecDirs of the warp's directions at a time: record (t, j) at
-    // (t * kGrRecDirs + j % kGrRecDirs) * kGrRecWords.
-    float* rec = rec_all + e * (4 * kGrRecDirs * kGrRecWords);
-    float* rec_t = rec + tl * kGrRecDirs * kGrRecWords;  // this lane's timestep
+    // Records of kGrRecDirs of the warp's directions at a time.
+    float* rec = rec_all + e * (4 * kGrRecStep);
+    float* rec_t = rec + tl * kGrRecStep;  // this lane's timestep
     uint32_t blk = 0;
     bool ok = true;
     for (int sl = blockIdx.x; ok; sl += gridDim.x) {
@@ -966,43 +987,41 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
                 for (int jj = 0; jj < 2; ++jj) {
                   const int j = hr + ps + 8 * jj;
                   grid_record<W>(p, x, tab, I.dir0 + dbase + min(j, nd - 1), j < nd, rval, n, c0, I.lbase, r0,
-                                 w.npass, rec_t + (ps + 8 * jj) * kGrRecWords);
+                                 w.npass, rec_t, ps + 8 * jj);
                 }
                 __syncwarp();
               }
 #pragma unroll
               for (int jb = hr; jb < hr + kGrRecDirs; jb += kGrBatch) {
                 if (jb >= nd) break;  // the same in every lane
-                // The batch's directions that read this pass with one shared load (codes are the
-                // same in every lane for those): loads and one wait per pair, then their sums.
-                const float* rb = rec_t + (jb - hr) * kGrRecWords;
+                // The batch's directions that read this pass with one shared load (codes are the same in every
+                // lane for those).  A direction's taps load while the previous one's are summed.
                 uint32_t col[kGrBatch];
                 int code[kGrBatch];
                 int live = 0;
 #pragma unroll
                 for (int bb = 0; bb < kGrBatch; ++bb) {
-                  code[bb] = __float_as_int(rb[bb * kGrRecWords + kGrCodeWord]);
+                  code[bb] = __float_as_int(rec_t[grid_rec_row(jb - hr + bb, kGrCodeWord / 4) + kGrCodeWord % 4]);
                   const bool use = code[bb] >= 0 && !(code[bb] & kGrWide) && ((code[bb] >> 8) & 255) == pp;
                   col[bb] = use ? 2u * static_cast<uint32_t>(code[bb] & 255) : 0u;
                   live |= (use ? 1 : 0) << bb;
                 }
                 float gs[kGrBatch] = {0.f, 0.f, 0.f, 0.f};
+                if (live) {
+                  uint32_t v[2][kGrLoadRegs];
+                  grid_load_start(tbase + col[0], v[0]);
 #pragma unroll
-                for (int bp = 0; bp < kGrBatch; bp += 2) {
-                  if ((live >> bp) & 3) {
-                    uint32_t v[2][kGrLoadRegs];
-                    grid_load_pair(tbase, col[bp], col[bp + 1], v);
-#pragma unroll
-                    for (int bb = 0; bb < 2; ++bb) {
-                      const float gsum = grid_tap_combine<W>(v[bb], rb + (bp + bb) * kGrRecWords, sgn);
-                      gs[bp + bb] = ((live >> (bp + bb)) & 1) ? gsum : 0.f;
-                    }
+                  for (int bb = 0; bb < kGrBatch; ++bb) {
+                    grid_load_wait(v[bb & 1]);
+                    if (bb + 1 < kGrBatch) grid_load_start(tbase + col[bb + 1], v[(bb + 1) & 1]);
+                    const float gsum = grid_tap_combine<W>(v[bb & 1], rec_t, jb - hr + bb, sgn);
+                    gs[bb] = ((live >> bb) & 1) ? gsum : 0.f;
                   }
                 }
 #pragma unroll
                 for (int bb = 0; bb < kGrBatch; ++bb)
                   if (code[bb] >= 0 && (code[bb] & kGrWide))  // the kGrWide bit is the same in every lane
-                    gs[bb] += grid_wide_sum<W>(rec + (jb - hr + bb) * kGrRecWords, tbase, sgn, tl, pp);
+                    gs[bb] += grid_wide_sum<W>(rec, jb - hr + bb, tbase, sgn, tl, pp);
                 acc[jb / kGrBatch] = fmaf(sc, grid_sum_timesteps(gs, tl), acc[jb / kGrBatch]);
               }
             }
