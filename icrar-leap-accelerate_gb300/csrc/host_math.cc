@@ -356,7 +356,8 @@ float grid_table(int32_t C, int32_t taps, double beta, int32_t lbase, int32_t ro
   int e = 0;
   (void)std::frexp(emax, &e);
   const double scale = std::ldexp(1.0, 14 - e);
-  out.assign(static_cast<size_t>(nchunk) * 2 * 2 * nrg * 128, 0);
+  const int nseg = (nchunk + 3) / 4;
+  out.assign(static_cast<size_t>(nseg) * 2 * nrg * 4 * 2 * 128, 0);
   const double kTwoPiD = 6.283185307179586476925286766559;
   for (int c = 0; c < C; ++c) {
     const int k = c - c0;
@@ -373,9 +374,9 @@ float grid_table(int32_t C, int32_t taps, double beta, int32_t lbase, int32_t ro
         const uint16_t lo = to_f16_bits(v[ri] - from_f16_bits(hi));
         const int rr = 2 * r + ri;  // re and im rows of a grid point are neighbours
         for (int hl = 0; hl < 2; ++hl) {
-          const size_t base = (static_cast<size_t>(q * 2 + hl) * 2 * nrg) * 128;
-          // The kernel's K-major 16-bit block layout (grid_f16_offset), in 2-byte units.
-          out[base + ((rr >> 3) * 2 + (kk >> 3)) * 64 + (rr & 7) * 8 + (kk & 7)] = hl == 0 ? hi : lo;
+          // K-major core matrices of 8 rows x 16 bytes, in 2-byte units.
+          const size_t block = (static_cast<size_t>(q / 4) * 2 * nrg + (rr >> 3)) * 8 + (q % 4) * 2 + hl;
+          out[block * 128 + (kk >> 3) * 64 + (rr & 7) * 8 + (kk & 7)] = hl == 0 ? hi : lo;
         }
       }
     }

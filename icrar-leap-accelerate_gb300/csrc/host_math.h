@@ -36,8 +36,9 @@ int pseudo_inverse(const double* A, int32_t m, int32_t n, double* Ad, std::strin
 // r in [0, rows), with Psi the Fourier transform of the exponential-of-semicircle
 // kernel of width `taps` and shape `beta` at frequency k / (2C).  Scaled by a power of
 // two (its largest entry in [2^13, 2^14)) and written as FP16 (hi, lo) splits in the
-// K-major layout the kernel copies from: [chunk of 16 channels][hi, lo][row group of 8]
-// [2 k-halves][8 rows x 8 k], rows 2 l + (0: re, 1: im).  Returns the inverse scale.
+// K-major layout the kernel copies from: [segment of 64 channels][row group of 8][chunk of 16
+// channels][hi, lo][2 k-halves][8 rows x 8 k], rows 2 l + (0: re, 1: im), the last segment filled up
+// with zeros.  Returns the inverse scale.
 float grid_table(int32_t C, int32_t taps, double beta, int32_t lbase, int32_t rows, std::vector<uint16_t>& out);
 
 // Interpolation weights of the gridded rotate + average as polynomials: for m = 0 .. taps-1,

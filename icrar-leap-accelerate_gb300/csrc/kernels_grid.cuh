@@ -53,15 +53,14 @@
 // Operands.  The tile's visibilities reach shared memory already scaled and split into
 // FP16 hi and lo parts in the MMA's canonical K-major layout: grid_split_operand builds
 // that copy of an integration once (8 KB per tile and 16-channel chunk, the bytes of the
-// visibilities), and each chunk is then one bulk copy, so no warp converts operands
-// between the copy and the MMAs.
+// visibilities), so no warp converts operands between the copy and the MMAs.
 //
 // Warp roles (14 warps): 0 = producer (bulk copies of the split operand and of the E
 // window), 1 = MMA issuer (+ TMEM owner), 2-5 = fold warps (add the finished hi*hi
 // segments and the corrections into the running sums), 6-13 = epilogue (warp w reads
 // TMEM lanes 32 (w % 4) ..; two warps per quarter take 32 directions each).  One ring of
-// kGrStages stages of {A hi, A lo, E window}, handed over in rounds of kGrMacro (one 64-channel
-// segment) and released by one MMA commit per round.  A round issues its 8 correction MMAs
+// kGrStages stages of {A hi, A lo, E window}, copied and handed over in rounds of kGrMacro (one
+// 64-channel segment) and released by one MMA commit per round.  A round issues its 8 correction MMAs
 // before its 4 hi*hi MMAs, so the fold that frees IS overlaps the corrections (a round's
 // stages all land before it starts).  Every wait is bounded; a timeout sets the error word, stops every
 // role, and the block still waits (bounded) for its copies and MMAs and frees its TMEM.
@@ -97,10 +96,14 @@ constexpr int kGrWarps = 6 + kGrEpiWarps;
 constexpr int kGrThreads = kGrWarps * 32;
 constexpr int kGrAHalf = 128 * kGrChunk * 2;            // one split of A: 128 rows x 16 f16 (32 B)
 constexpr int kGrOpBytes = 2 * kGrAHalf;                 // hi + lo of one chunk of one tile
-constexpr int kGrEBytes = 2 * 2 * kGrJwMax * kGrChunk * 2;  // [hl][2 Jw rows x 32 B]
-// Stage: [A hi][A lo][E hi][E lo]
-constexpr int kGrStageBytes = kGrOpBytes + kGrEBytes;
-constexpr int kGrEOffset = kGrOpBytes;
+// A round's stages in shared memory: [A of its 4 chunks: hi, lo each][E window: row groups of 8 rows, in each the 4
+// chunks' hi and lo, 256 bytes apiece].  The operand and the grid matrix have the same order in memory, so a round
+// is two bulk copies.  (Against one copy per chunk and half, 12 a round: 17.55 -> 17.26 ms at 131328 rows, where a
+// unit's tiles are few; 128 antennas 694.6 -> 693.5 us.)
+constexpr int kGrEGroup = kGrMacro * 2 * 256;            // one group of 8 E rows of a segment
+constexpr int kGrABytes = kGrMacro * kGrOpBytes;
+constexpr int kGrEBytes = 2 * kGrJwMax / 8 * kGrEGroup;
+constexpr int kGrRoundBytes = kGrABytes + kGrEBytes;
 constexpr int kGrRecWords = 16;                          // per (direction, timestep) record: 4 16-byte rows
 constexpr int kGrCodeWord = kGrTaps + 3;                 // record: W + 1 weights, cr, sr, then the load code
 constexpr int kGrRecDirs = 16;                           // directions whose records a warp holds at a time
@@ -108,7 +111,7 @@ constexpr int kGrRecDirs = 16;                           // directions whose rec
 // the 4 timesteps of a warp's lanes read one row of a direction from different banks, and the rows of a record are
 // exchanged with its direction's bits 1 and 2, so that the 8 lanes of a timestep write one row of theirs without
 // conflicts either.  (Without both the records took 7 to 9 of a tile's 17 thousand cycles of shared memory, beside 4
-// of the MMAs' operands and 2.7 of the copies: the bound of the kernel.  128 antennas: REC0 -> REC1 ms a call.)
+// of the MMAs' operands and 2.7 of the copies: the bound of the kernel.  A 128-antenna call: 761 -> 726 us.)
 constexpr int kGrRecStep = kGrRecDirs * kGrRecWords + 4;  // words per timestep
 constexpr int kGrRecBytes = kGrEpiWarps * 4 * kGrRecStep * 4;
 __host__ __device__ constexpr int grid_rec_row(int j, int i) { return j * kGrRecWords + ((i ^ ((j >> 1) & 3)) << 2); }
@@ -126,7 +129,7 @@ static_assert(kGrTaps + 1 <= kGrLoadCols, "one load per stencil");
 static_assert(kGrCodeWord < kGrRecWords, "record layout");
 
 __host__ __device__ constexpr int grid_smem_bytes() {
-  return kGrStages * kGrStageBytes + kTwiddleSize * 8 + kGrRecBytes + kGrNumBars * 8 + 16;
+  return kGrMacroStages * kGrRoundBytes + kTwiddleSize * 8 + kGrRecBytes + kGrNumBars * 8 + 16;
 }
 static_assert(grid_smem_bytes() <= 227 * 1024, "one block's dynamic shared memory (227 KB on sm_103)");
 
@@ -134,6 +137,7 @@ static_assert(grid_smem_bytes() <= 227 * 1024, "one block's dynamic shared memor
 __host__ __device__ constexpr int grid_lbase(int C) { return ((C + kGrTaps + 8 + 7) / 8) * 8; }
 __host__ __device__ constexpr int grid_rows(int C) { return ((grid_lbase(C) + C + kGrJwMax + 8 + 7) / 8) * 8; }
 __host__ __device__ constexpr int grid_chunks(int C) { return (C + kGrChunk - 1) / kGrChunk; }
+__host__ __device__ constexpr int grid_segments(int C) { return (grid_chunks(C) + kGrSegChunks - 1) / kGrSegChunks; }
 // Split grid operand of an integration: per (quad, timestep block, 16-channel chunk) the
 // tile's scaled visibilities as FP16 hi and lo parts in the MMA's canonical K-major layout,
 // [hi: 16 row groups x 2 k-halves x 8 rows x 16 B][lo: the same], 8 KB, exactly what the
@@ -161,8 +165,8 @@ __host__ __device__ constexpr int grid_f16_offset(int row, int k) {
 // Bound by HBM: the visibilities read once, the operand (as many bytes) written.  A lane reads 16 bytes, two pols of
 // (timestep lane / 8, baseline (lane / 2) % 4), and writes 64-byte runs of the operand, 8 channels of its 4 rows;
 // the second pass over the tile (after the maxima) finds it in L2: kGrSplitBlocks blocks per SM hold 152 x 2 x
-// 192 KB = 60 MB at 384 channels, and the operand's lines are written evict-first (3 blocks per SM: 0.8 ms).  (4-byte lanes, one channel at a time: 856 us for the 128-antenna integration of
-// 1.42 GB, 510 us now.)
+// 192 KB = 60 MB at 384 channels, and the operand's lines are written evict-first (3 blocks per SM: 0.8 ms).  For
+// the 128-antenna integration of 1.42 GB, 510 us; with 4-byte lanes, one channel at a time, 856 us.
 constexpr int kGrSplitThreads = 512;
 constexpr int kGrSplitBlocks = 2;  // per SM
 static __global__ void __launch_bounds__(kGrSplitThreads, kGrSplitBlocks)
@@ -696,7 +700,9 @@ __device__ __forceinline__ void grid_flush(const float (&acc)[kGrWarpDirs / kGrB
   }
 }
 
-// One lane of a converged warp, the same in every call.
+// One lane of a converged warp, the same in every call.  With it, and with loop bounds that the compiler knows to be
+// uniform (grid_uniform), the MMA warp issues its instructions without a divergence check around each: a 128-antenna
+// call 772 -> 761 us.
 __device__ __forceinline__ bool grid_elect() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -710,8 +716,8 @@ template <int W>
 __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const GridParams p) {
   extern __shared__ __align__(128) unsigned char grid_smem[];
   unsigned char* smem = grid_smem;
-  unsigned char* ve = smem;                                          // [kGrStages][V then A hi | A lo | E]
-  float2* tab = reinterpret_cast<float2*>(smem + kGrStages * kGrStageBytes);
+  unsigned char* ve = smem;                                          // [kGrMacroStages][A | E]
+  float2* tab = reinterpret_cast<float2*>(smem + kGrMacroStages * kGrRoundBytes);
   float* rec_all = reinterpret_cast<float*>(tab + kTwiddleSize);
   uint64_t* bars = reinterpret_cast<uint64_t*>(rec_all + kGrRecBytes / 4);
   uint64_t* vfull = bars;                      // [kGrMacroStages] bytes of a round's stages landed
@@ -760,33 +766,31 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
         const GridUnit g = grid_unit(p, u);
         const GridItem& I = p.items[g.item];
         const GridWindow w = p.win[u];
-        for (int tb = 0; tb < g.ntb && ok; ++tb)
-          for (int ps = 0; ps < w.npass && ok; ++ps)
-            for (int q0 = 0; q0 < I.nchunk; q0 += kGrMacro, ++ctr) {
+        const int nchunk = I.nchunk;
+        const int64_t eseg = static_cast<int64_t>(2 * I.nrg) * kGrEGroup;  // a segment of the grid matrix
+        // The tile's operand: tiles of a unit follow one another (timestep blocks t_lo / 4 ..).
+        const unsigned char* asrc =
+            I.op + (static_cast<int64_t>(g.quad) * I.ntb + g.t_lo / 4) * nchunk * kGrOpBytes;
+        for (int tb = 0; tb < g.ntb && ok; ++tb, asrc += static_cast<int64_t>(nchunk) * kGrOpBytes)
+          for (int ps = 0; ps < w.npass && ok; ++ps) {
+            const unsigned char* esrc = I.etab + static_cast<int64_t>(2 * (w.rg0 + ps * (kGrPassStride / 8))) * kGrEGroup;
+            for (int q0 = 0; q0 < nchunk; q0 += kGrMacro, ++ctr) {
               const int m = ctr % kGrMacroStages;
-              const int nq = min(kGrMacro, I.nchunk - q0);
+              const int nq = min(kGrMacro, nchunk - q0);
               if (ctr >= kGrMacroStages && !grid_wait(&sdone[m], ((ctr / kGrMacroStages) - 1) & 1, abort_flag)) {
                 grid_fail(p, abort_flag);
                 ok = false;
                 break;
               }
-              mbar_arrive_expect_tx(&vfull[m], nq * (kGrOpBytes + 4 * w.jw * 32));
-              const int rg = w.rg0 + ps * (kGrPassStride / 8);
-              const int tbi = g.t_lo / 4 + tb;  // the tile's timestep block in the integration
-              for (int i = 0; i < nq; ++i) {
-                const int q = q0 + i;
-                unsigned char* st = ve + (m * kGrMacro + i) * kGrStageBytes;
-                // The chunk's A operand, hi and lo, already in the MMA layout.
-                bulk_copy_g2s(st, I.op + ((static_cast<int64_t>(g.quad) * I.ntb + tbi) * I.nchunk + q) * kGrOpBytes,
-                              kGrOpBytes, &vfull[m]);
-#pragma unroll
-                for (int hl = 0; hl < 2; ++hl) {
-                  // Window grid points [8 rg, 8 rg + jw): 2 jw interleaved (re, im) rows.
-                  const unsigned char* src = I.etab + (static_cast<int64_t>(q * 2 + hl) * 2 * I.nrg + 2 * rg) * 256;
-                  bulk_copy_g2s(st + kGrEOffset + hl * 2 * w.jw * 32, src, 2 * w.jw * 32, &vfull[m]);
-                }
-              }
+              // The chunks' A operands, hi and lo, already in the MMA layout, and the window's E rows (grid points
+              // [8 rg, 8 rg + jw): 2 jw interleaved (re, im) rows).
+              const uint32_t abytes = nq * kGrOpBytes, ebytes = (w.jw >> 2) * kGrEGroup;
+              mbar_arrive_expect_tx(&vfull[m], abytes + ebytes);
+              unsigned char* st = ve + m * kGrRoundBytes;
+              bulk_copy_g2s(st, asrc + static_cast<int64_t>(q0) * kGrOpBytes, abytes, &vfull[m]);
+              bulk_copy_g2s(st + kGrABytes, esrc + static_cast<int64_t>(q0 / kGrMacro) * eseg, ebytes, &vfull[m]);
             }
+          }
       }
       // Do not leave while copies issued by this block may still land.
       for (uint32_t j = (ctr > kGrMacroStages ? ctr - kGrMacroStages : 0); j < ctr; ++j)
@@ -800,7 +804,7 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
     uint32_t ctr = 0, blk = 0, mids = 0;
     bool ok = true, issued = false;
     const uint64_t adesc0 = tc_smem_desc(ve, kTcLbo, kTcSbo);
-    const uint64_t edesc0 = tc_smem_desc(ve + kGrEOffset, kTcLbo, kTcSbo);
+    const uint64_t edesc0 = tc_smem_desc(ve + kGrABytes, kTcLbo, kGrEGroup);
     for (int sl = blockIdx.x; ok; sl += gridDim.x) {
       const int u = grid_uniform(sl < p.nslots ? __ldg(p.order + sl) : -1);
       if (u < 0) break;
@@ -808,7 +812,6 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
       const int ntb = grid_uniform(g.ntb), nchunk = grid_uniform(p.items[g.item].nchunk);
       const int jw = grid_uniform(p.win[u].jw), npass = grid_uniform(p.win[u].npass);
       const uint32_t idesc = grid_idesc_f16(128, 2 * jw);
-      const uint64_t elo = static_cast<uint64_t>(2 * jw * 2);  // E lo after E hi, in descriptor units of 16 bytes
       for (int tb = 0; tb < ntb && ok; ++tb)
         for (int ps = 0; ps < npass && ok; ++ps, ++blk) {
           const uint32_t b = blk & 1;
@@ -832,16 +835,17 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
             // A round is one segment.  Its correction MMAs go first: they give the fold of the
             // previous segment time to finish before the hi*hi MMAs restart IS.
             const int seg = q0 / kGrSegChunks;
-            // Descriptors of stage i: A hi/lo at +0 / +kGrAHalf, E hi/lo at +0 / +2*jw*32 from their
-            // bases (address field >> 4).
-            constexpr uint64_t sst = static_cast<uint64_t>(kGrStageBytes >> 4);
-            const uint64_t ad = adesc0 + m * (kGrMacro * sst), ed = edesc0 + m * (kGrMacro * sst);
+            // Descriptors of chunk i (address field >> 4): A hi/lo at i kGrOpBytes (+ kGrAHalf), E hi/lo at
+            // i 512 (+ 256), row groups kGrEGroup apart.
+            constexpr uint64_t ast = kGrOpBytes >> 4, est = 512 >> 4;
+            const uint64_t ad = adesc0 + m * static_cast<uint64_t>(kGrRoundBytes >> 4);
+            const uint64_t ed = edesc0 + m * static_cast<uint64_t>(kGrRoundBytes >> 4);
             if (lead) {
 #pragma unroll
               for (int i = 0; i < kGrMacro; ++i)
                 if (i < nq)
-                  grid_mma_corrections(tmem + kGrAC, ad + i * sst, ad + i * sst + (kGrAHalf >> 4), ed + i * sst,
-                                       ed + i * sst + elo, idesc, q0 + i > 0 ? 1u : 0u);
+                  grid_mma_corrections(tmem + kGrAC, ad + i * ast, ad + i * ast + (kGrAHalf >> 4), ed + i * est,
+                                       ed + i * est + (256 >> 4), idesc, q0 + i > 0 ? 1u : 0u);
             }
             issued = true;
             if (seg >= 2 && !grid_wait(is_empty, (mids - 1) & 1, abort_flag)) {
@@ -852,7 +856,7 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
               if (lead) {
 #pragma unroll
                 for (int i = 0; i < kGrMacro; ++i)
-                  if (i < nq) grid_mma_hihi(dst, ad + i * sst, ed + i * sst, idesc, i > 0 ? 1u : 0u);
+                  if (i < nq) grid_mma_hihi(dst, ad + i * ast, ed + i * est, idesc, i > 0 ? 1u : 0u);
               }
               if (seg >= 1 && q0 + nq < nchunk) ++mids;  // a middle segment, folded
             }
@@ -956,6 +960,11 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
         const float sc =
             __ldg(I.vinv + (static_cast<int64_t>(g.quad) * I.ntb + g.t_lo / 4 + tb) * 16 + quarter * 4 + (ps >> 1)) *
             I.einv;
+        // The row's split UVWs, on their way while the tile's sums are waited for (698 -> 694 us; 131328 rows:
+        // 17.95 -> 17.55 ms).
+        float x[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) x[i] = __ldg(I.uvw_f + 6 * r + i);
         for (int pp = 0; pp < w.npass; ++pp, ++blk) {
           const uint32_t rb = blk & 1;
           if (!grid_wait(&rs_full[rb], (blk >> 1) & 1, abort_flag)) {
@@ -978,10 +987,7 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
               {
                 // Lane (t, ps) computes the records of directions hr + ps and hr + 8 + ps at
                 // timestep t; the records past nd say "no load".  (Written as a loop, the two
-                // records take fewer registers than two inlined calls: the kernel does not spill.)
-                float x[6];
-#pragma unroll
-                for (int i = 0; i < 6; ++i) x[i] = __ldg(I.uvw_f + 6 * r + i);
+                // records take fewer registers than two inlined calls, which spilt.)
                 __syncwarp();
 #pragma unroll 1
                 for (int jj = 0; jj < 2; ++jj) {
@@ -995,7 +1001,8 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
               for (int jb = hr; jb < hr + kGrRecDirs; jb += kGrBatch) {
                 if (jb >= nd) break;  // the same in every lane
                 // The batch's directions that read this pass with one shared load (codes are the same in every
-                // lane for those).  A direction's taps load while the previous one's are summed.
+                // lane for those).  A direction's taps load while the previous one's are summed (a 128-antenna
+                // call: 726 -> 698 us; loads of the next batch before this one's end spill: 854 us).
                 uint32_t col[kGrBatch];
                 int code[kGrBatch];
                 int live = 0;
