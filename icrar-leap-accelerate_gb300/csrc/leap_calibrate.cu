@@ -903,8 +903,17 @@ int autotune_batch(leap_ctx* ctx, const std::vector<WorkItem>& items, int32_t D,
     max_ndir = std::max(max_ndir, w.ndir);
   }
   std::vector<TuneChoice> cands;
-  for (int tpb : {pipe_tiles(max_ndir), pipe_tiles(min_ndir)}) {
-    if (!cands.empty() && cands.back().tpb == tpb) continue;
+  // Fewer tiles per block give more units, which a small batch needs to fill the GPU (11 chunks of 1 or 2 timesteps,
+  // 33 antennas, 8 directions each: 140 us a call with 4 tiles, 126 with the better of 4 and 1).
+  int64_t units = 0;
+  const int64_t nbl = std::max<int64_t>(1, ctx->md.k.nbaselines);
+  const int most = pipe_tiles(max_ndir), dirs = kPipeNC / most * kPipeDPW;
+  for (const auto& w : items) {
+    auto it = ctx->integ.find(w.slot);  // (a missing one is refused by the first trial)
+    if (it != ctx->integ.end()) units += it->second.rows / nbl * ((nbl + 32 * most - 1) / (32 * most)) * ((w.ndir + dirs - 1) / dirs);
+  }
+  for (int tpb : {4, 2, 1}) {
+    if (tpb != most && tpb != pipe_tiles(min_ndir) && (tpb > 1 || units >= 4 * ctx->sms)) continue;
     for (int waves : {2, 4, 8}) cands.push_back(TuneChoice{tpb, waves, 0});
   }
   if (ctx->mma_rotate > 0 && precision == LEAP_PRECISION_MIXED && min_ndir >= 12)
