@@ -502,4 +502,59 @@ void fx_tables(std::vector<FxLimbs>& out) {
   }
 }
 
+// A run's units are dealt at once: block b takes those n_b of the costs load_b, load_b + cost, ... that are among the
+// `count` least of all blocks, the numbers that taking the least loaded block for each unit in turn gives (a heap of
+// blocks took 3.0 ms of the host for 65664 units and 102 us for 2064, this 78 and 8 us).
+void schedule_units(std::vector<UnitRun> runs, int32_t grid, std::vector<int32_t>& order) {
+  std::stable_sort(runs.begin(), runs.end(), [](const UnitRun& a, const UnitRun& b) { return a.cost > b.cost; });
+  std::vector<int64_t> load(grid, 0);
+  std::vector<int32_t> length(grid, 0), n(grid);
+  order.clear();
+  for (const UnitRun& r : runs) {
+    if (r.count <= 0) continue;
+    const int64_t cost = std::max<int64_t>(1, r.cost);
+    auto below = [&](int64_t x, int64_t l) { return x > l ? (x - l + cost - 1) / cost : 0; };
+    auto taken = [&](int64_t x) {
+      int64_t s = 0;
+      for (int64_t l : load) s += below(x, l);
+      return s;
+    };
+    // The largest x with at most `count` costs below it.
+    int64_t lo = *std::min_element(load.begin(), load.end()), hi = lo + (static_cast<int64_t>(r.count) + 1) * cost;
+    while (hi - lo > 1) {
+      const int64_t mid = lo + (hi - lo) / 2;
+      (taken(mid) <= r.count ? lo : hi) = mid;
+    }
+    int64_t rest = r.count, most = 0;
+    for (int32_t b = 0; b < grid; ++b) rest -= n[b] = static_cast<int32_t>(below(lo, load[b]));
+    for (int32_t b = 0; b < grid && rest > 0; ++b)
+      if (load[b] + n[b] * cost == lo) {
+        ++n[b];
+        --rest;
+      }
+    int64_t rounds = 0;
+    for (int32_t b = 0; b < grid; ++b) {
+      most = std::max<int64_t>(most, n[b]);
+      rounds = std::max<int64_t>(rounds, length[b] + n[b]);
+    }
+    if (static_cast<int64_t>(order.size()) < rounds * grid) order.resize(rounds * grid, -1);
+    // Neighbouring units to different blocks at the same time.
+    int32_t base = r.begin, in = 0;
+    for (int64_t k = 0; k < most; ++k)
+      for (int32_t b = 0; b < grid; ++b) {
+        if (n[b] <= k) continue;
+        order[static_cast<int64_t>(length[b] + k) * grid + b] = base + in;
+        if (++in == r.per) {
+          in = 0;
+          base += r.stride;
+        }
+      }
+    for (int32_t b = 0; b < grid; ++b) {
+      load[b] += n[b] * cost;
+      length[b] += n[b];
+    }
+  }
+  order.resize(order.size() + grid, -1);
+}
+
 }  // namespace leapgb

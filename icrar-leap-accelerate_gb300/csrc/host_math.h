@@ -60,4 +60,14 @@ bool fx_spectrum(double f0, double df, int32_t channels, const double* lambda, F
 // The two phasor tables: kFxTable entries exp(2 pi i j / 2^10), then kFxTable of exp(2 pi i j / 2^20).
 void fx_tables(std::vector<FxLimbs>& out);
 
+// `count` units of equal cost for schedule_units: numbers begin + (i / per) * stride + i % per, i < count.
+struct UnitRun {
+  int64_t cost;
+  int32_t begin, count, per, stride;
+};
+
+// Unit schedule of a persistent kernel with `grid` blocks: longest unit first, each to the least loaded block.
+// order[k * grid + b] is the k-th unit of block b, or -1 after its last; the last round is all -1.
+void schedule_units(std::vector<UnitRun> runs, int32_t grid, std::vector<int32_t>& order);
+
 }  // namespace leapgb

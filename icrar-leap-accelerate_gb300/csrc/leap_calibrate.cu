@@ -64,6 +64,13 @@ int dispatch_fixed(leap_ctx* ctx, int32_t vis_type, const FxArgs& fa, int nw, di
                                          : launch_fixed<double2, 4>(ctx, fa, nw, grid, s);
 }
 
+// The units of an item, `groups` times `nslab` timestep slabs: all slabs cost the same but the last.
+template <typename Cost>
+void push_unit_runs(std::vector<UnitRun>& runs, int begin, int groups, int nslab, Cost cost) {
+  if (nslab > 1) runs.push_back(UnitRun{cost(0), begin, groups * (nslab - 1), nslab - 1, nslab});
+  runs.push_back(UnitRun{cost(nslab - 1), begin + nslab - 1, groups, 1, nslab});
+}
+
 // Grid matrix of the gridded kernel for C channels (built once per channel count) and the
 // inverse of its scale.
 const unsigned char* grid_table_for(leap_ctx* ctx, int C, float& einv) {
@@ -173,36 +180,17 @@ int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const doubl
       it.out = ctx->avg.as<double2>() + static_cast<int64_t>(it.dir0) * 4 * nbl;
     }
   }
-  // Longest unit first, each to the least-loaded block (cost: timestep blocks x chunks).
+  // Cost of a unit: timestep blocks x chunks.
   const int grid = std::min(units, ctx->sms);
   {
-    std::vector<std::pair<int64_t, int>> cost;
-    cost.reserve(units);
-    for (const GridItem& it : git) {
-      const int per_item = it.nquad * it.uparts * it.nslab;
-      for (int l = 0; l < per_item; ++l) {
-        const int slab = l % it.nslab;
+    std::vector<UnitRun> runs;
+    for (const GridItem& it : git)
+      push_unit_runs(runs, it.unit_begin, it.nquad * it.uparts, it.nslab, [&](int slab) {
         const int t_lo = slab * it.tb_per_slab * 4, t_hi = std::min(it.T, t_lo + it.tb_per_slab * 4);
-        cost.emplace_back(-static_cast<int64_t>((t_hi - t_lo + 3) / 4) * (it.nchunk + 2 * it.udg),
-                          it.unit_begin + l);
-      }
-    }
-    std::stable_sort(cost.begin(), cost.end());
-    std::vector<std::vector<int32_t>> lists(grid);
-    std::priority_queue<std::pair<int64_t, int>, std::vector<std::pair<int64_t, int>>, std::greater<>> load;
-    for (int b = 0; b < grid; ++b) load.emplace(0, b);
-    for (const auto& c : cost) {
-      auto [l, b] = load.top();
-      load.pop();
-      lists[b].push_back(c.second);
-      load.emplace(l - c.first, b);
-    }
-    size_t rounds = 0;
-    for (const auto& l : lists) rounds = std::max(rounds, l.size());
+        return static_cast<int64_t>((t_hi - t_lo + 3) / 4) * (it.nchunk + 2 * it.udg);
+      });
     std::vector<int32_t>& order = ctx->grid_order_host;
-    order.assign(rounds * grid + grid, -1);
-    for (int b = 0; b < grid; ++b)
-      for (size_t k = 0; k < lists[b].size(); ++k) order[k * grid + b] = lists[b][k];
+    schedule_units(std::move(runs), grid, order);
     LEAP_CUDA(ctx->grid_order.ensure(sizeof(int32_t) * order.size()), "alloc unit order");
     if (!ctx->capturing)
       LEAP_CUDA(cudaMemcpyAsync(ctx->grid_order.ptr, order.data(), sizeof(int32_t) * order.size(),
@@ -411,38 +399,20 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
         it.out = ctx->avg.as<double2>() + static_cast<int64_t>(it.dir0) * 4 * nbl;
       }
     }
-    // Unit schedule: longest unit first, each to the least-loaded block (cost in channel
-    // steps: timesteps x (padded channels + a per-timestep set-up allowance)).
+    // Cost of a unit in channel steps: timesteps x (padded channels + a per-timestep set-up allowance).
     const int grid = std::min(units, ctx->sms);
     {
       const int CH = PipeShape<1>::CH;
-      std::vector<std::pair<int64_t, int>> cost;
-      cost.reserve(units);
+      std::vector<UnitRun> runs;
       for (const PipeItem& it : pit) {
         const int64_t per_t = static_cast<int64_t>((it.C + CH - 1) / CH) * CH + 8;
-        const int per_item = it.tgroups * it.dgroups * it.nslab;
-        for (int l = 0; l < per_item; ++l) {
-          const int slab = l % it.nslab;
+        push_unit_runs(runs, it.unit_begin, it.tgroups * it.dgroups, it.nslab, [&](int slab) {
           const int t_lo = slab * it.t_per_slab, t_hi = std::min(it.T, t_lo + it.t_per_slab);
-          cost.emplace_back(-(t_hi - t_lo) * per_t, it.unit_begin + l);
-        }
+          return (t_hi - t_lo) * per_t;
+        });
       }
-      std::stable_sort(cost.begin(), cost.end());
-      std::vector<std::vector<int32_t>> lists(grid);
-      std::priority_queue<std::pair<int64_t, int>, std::vector<std::pair<int64_t, int>>, std::greater<>> load;
-      for (int b = 0; b < grid; ++b) load.emplace(0, b);
-      for (const auto& c : cost) {
-        auto [l, b] = load.top();
-        load.pop();
-        lists[b].push_back(c.second);
-        load.emplace(l - c.first, b);
-      }
-      size_t rounds = 0;
-      for (const auto& l : lists) rounds = std::max(rounds, l.size());
       std::vector<int32_t>& order = ctx->pipe_order_host;
-      order.assign(rounds * grid + grid, -1);  // one extra round of -1 ends every block
-      for (int b = 0; b < grid; ++b)
-        for (size_t k = 0; k < lists[b].size(); ++k) order[k * grid + b] = lists[b][k];
+      schedule_units(std::move(runs), grid, order);
       LEAP_CUDA(ctx->pipe_order.ensure(sizeof(int32_t) * order.size()), "alloc unit order");
       if (!ctx->capturing)
         LEAP_CUDA(cudaMemcpyAsync(ctx->pipe_order.ptr, order.data(), sizeof(int32_t) * order.size(),
