@@ -354,16 +354,19 @@ __device__ __forceinline__ void grid_fail(const GridParams& p, volatile int* abo
 // direction groups.  One 64-thread block per unit: thread r takes rows r, r + 64, ... of the
 // unit (baseline r % 4 of the quad, timestep t_lo + r / 4), loads its UVWs once and walks the
 // directions, whose slopes the block stages in shared memory 64 at a time.
+//
+// The grid point below a position grows with the slope, so only the least and the largest slope of the unit are
+// rounded.  They are taken in plain FP32, and in the double-float arithmetic of the records only for a unit where the
+// error of FP32 leaves one of the two grid points open or a slope may wrap at half a turn (one in a few
+// thousand).  That leaves 14 instructions a slope and no conversion (16 lanes per clock); with the records' arithmetic and a
+// rounding for each slope: 408 us for 65664 units of 64 rows and 64 directions, 199 now
+// (2 or 4 threads per row: 230 and 315, the blocks' own latency counts).
 constexpr int kGrWinThreads = 64;
-static __global__ void __launch_bounds__(kGrWinThreads) grid_windows(const GridParams p) {
-  __shared__ float kbs[kGrDirs][6];
-  __shared__ int red[2][kGrWinThreads / 32];
-  const int u = blockIdx.x;
-  const GridUnit g = grid_unit(p, u);
-  const GridItem& I = p.items[g.item];
-  const int n = 2 * I.C;
+
+template <typename Slope>
+__device__ __forceinline__ void grid_each_slope(const GridParams& p, const GridUnit& g, const GridItem& I,
+                                                float (*kbs)[6], Slope slope) {
   const int nrow = (g.t_hi - g.t_lo) * 4;
-  int smin = 0x7fffffff, smax = -0x7fffffff;
   for (int dg = g.dg_lo; dg < g.dg_hi; ++dg) {
     const int nd = min(kGrDirs, I.ndir - dg * kGrDirs);
     __syncthreads();  // the previous group's slopes are no longer read
@@ -377,28 +380,81 @@ static __global__ void __launch_bounds__(kGrWinThreads) grid_windows(const GridP
       float x[6];
 #pragma unroll
       for (int i = 0; i < 6; ++i) x[i] = __ldg(I.uvw_f + 6 * r + i);
-      for (int d = 0; d < nd; ++d) {
-        float f;
-        const int i0 = grid_position(df_dot3_turns_u32(kbs[d], x), n, f);
-        const int st = grid_stencil_start(i0, f);
-        smin = min(smin, st);
-        smax = max(smax, st);
-      }
+      for (int d = 0; d < nd; ++d) slope(kbs[d], x);
     }
   }
-  smin = __reduce_min_sync(0xffffffffu, smin);
-  smax = __reduce_max_sync(0xffffffffu, smax);
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = smin;
-    red[1][threadIdx.x >> 5] = smax;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+}
+
+static __global__ void __launch_bounds__(kGrWinThreads) grid_windows(const GridParams p) {
+  __shared__ float kbs[kGrDirs][6];
+  __shared__ float fred[3][kGrWinThreads / 32];
+  __shared__ int red[2][kGrWinThreads / 32];
+  const int u = blockIdx.x;
+  const GridUnit g = grid_unit(p, u);
+  const GridItem& I = p.items[g.item];
+  const int n = 2 * I.C, warp = threadIdx.x >> 5;
+  const float inf = __int_as_float(0x7F800000), fn = static_cast<float>(n);
+  float lo = inf, hi = -inf, mag = 0.f;
+  bool odd = false;
+  grid_each_slope(p, g, I, kbs, [&](const float* k, const float* x) {
+    const float pu = k[0] * x[0], pv = k[2] * x[2], pw = k[4] * x[4];
+    const float s = pu + pv + pw;
+    const float fr = s - ((s + 12582912.f) - 12582912.f);  // in [-1/2, 1/2] for |s| < 2^22
+    lo = fminf(lo, fr);
+    hi = fmaxf(hi, fr);
+    const float m = fabsf(pu) + fabsf(pv) + fabsf(pw);
+    mag = fmaxf(mag, m);
+    odd |= !(m < 4194304.f);  // or NaN
+  });
 #pragma unroll
-    for (int w = 1; w < kGrWinThreads / 32; ++w) {
+  for (int o = 16; o; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    mag = fmaxf(mag, __shfl_xor_sync(0xffffffffu, mag, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    fred[0][warp] = lo;
+    fred[1][warp] = hi;
+    fred[2][warp] = mag;
+  }
+  odd = __syncthreads_or(odd);
+#pragma unroll
+  for (int w = 0; w < kGrWinThreads / 32; ++w) {
+    lo = fminf(lo, fred[0][w]);
+    hi = fmaxf(hi, fred[1][w]);
+    mag = fmaxf(mag, fred[2][w]);
+  }
+  // A slope is off by less than e turns: five errors of 2^-24 of its products at most, and those of the lines below.
+  const float e = fmaf(mag, 0x1p-21f, 0x1p-22f);
+  const float flo = floorf((lo - e) * fn), fhi = floorf((hi + e) * fn);
+  int smin = 0x7fffffff, smax = -0x7fffffff;
+  if (!odd && lo > hi) {
+    // no row
+  } else if (!odd && lo - e > -0.5f && hi + e < 0.5f && flo == floorf((lo + e) * fn) && fhi == floorf((hi - e) * fn)) {
+    smin = grid_stencil_start(static_cast<int>(flo), 0.f);
+    smax = grid_stencil_start(static_cast<int>(fhi), 0.f);
+  } else {  // the same in the whole block
+    grid_each_slope(p, g, I, kbs, [&](const float* k, const float* x) {
+      float f;
+      const int i0 = grid_position(df_dot3_turns_u32(k, x), n, f);
+      const int st = grid_stencil_start(i0, f);
+      smin = min(smin, st);
+      smax = max(smax, st);
+    });
+    smin = __reduce_min_sync(0xffffffffu, smin);
+    smax = __reduce_max_sync(0xffffffffu, smax);
+    if ((threadIdx.x & 31) == 0) {
+      red[0][warp] = smin;
+      red[1][warp] = smax;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kGrWinThreads / 32; ++w) {
       smin = min(smin, red[0][w]);
       smax = max(smax, red[1][w]);
     }
+  }
+  if (threadIdx.x == 0) {
     GridWindow w{0, 16, 0, 0};
     if (smin <= smax) {
       w.rg0 = (smin + I.lbase) >> 3;
