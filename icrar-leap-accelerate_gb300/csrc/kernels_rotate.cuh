@@ -366,73 +366,6 @@ __global__ void __launch_bounds__(128) refant_average_fp64(RotateArgs a, const i
   }
 }
 
-// ---------------------------------------------------------------------------
-// Reference-antenna baselines in compensated FP32 (mixed form, complex<float>
-// input).  Same sums as refant_average_fp64, at about 1e-9 relative per term,
-// on the FP32 pipe (GB300's FP64 rate is ~1/70 of FP32):
-//  * phase: 64-bit fixed-point turns  pa + c*pb  (from FP64 A, B per timestep);
-//  * twiddle: the top 10 bits pick a (cos, sin) entry held as (hi, lo) float
-//    pairs (df_tab), the next 24 bits give delta < 2*pi/1024, and
-//    z = entry * (1 - delta^2/2 + i*(delta - delta^3/6)) is formed as entry_hi
-//    plus a correction (absolute error ~5e-10) and renormalised with TwoSum so
-//    that the low part is below one FP32 ulp;
-//  * product v*z_hi is exact (TwoProd), v*z_lo is rounded (error <= 4e-10 |v|),
-//    and the running sum is a TwoSum pair, so the sum carries no FP32 rounding;
-//  * a warp's two directions run as the two halves of paired FP32 instructions
-//    (FFMA2, FADD2, FMUL2), which round each half exactly as the scalar
-//    operation; a - b is formed as fma(b, -1, a) (one rounding, as the
-//    subtraction) and a negated product as fma(a, -b, c) = fma(-a, b, c), so
-//    each half carries the scalar sequence's sums bit for bit, at about half
-//    the instructions.
-// ---------------------------------------------------------------------------
-struct DfAcc2 {
-  float2 s, c;  // value = s + c, one direction per half
-};
-
-__device__ __forceinline__ float2 df_sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
-
-__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& e) {
-  s = __fadd2_rn(a, b);
-  const float2 bb = df_sub2(s, a);
-  e = __fadd2_rn(df_sub2(a, df_sub2(s, bb)), df_sub2(b, bb));
-}
-
-// acc += x * (yh + yl) per half (nx = -x): x*yh = p + e exactly (TwoProd), TwoSum of
-// acc.s and p, and err + (x*yl + e) into acc.c.
-__device__ __forceinline__ void df_add_product2(DfAcc2& acc, float2 x, float2 nx, float2 yh, float2 yl) {
-  const float2 p = __fmul2_rn(x, yh);
-  const float2 en = __ffma2_rn(nx, yh, p);  // p - x*yh = -e, exact
-  float2 sum, err;
-  two_sum2(acc.s, p, sum, err);
-  acc.s = sum;
-  acc.c = __fadd2_rn(acc.c, df_sub2(err, __ffma2_rn(nx, yl, en)));  // -(x*yl + e) from nx, en
-}
-
-// Twiddles of two phases (one per half) as (hi, lo) pairs.
-__device__ __forceinline__ void df_twiddle2(uint64_t t0, uint64_t t1, const float4* __restrict__ tab, float2& zrh,
-                                            float2& zrl, float2& zih, float2& zil) {
-  const float4 a = tab[t0 >> 54], b = tab[t1 >> 54];  // (cos_hi, cos_lo, sin_hi, sin_lo)
-  const float2 tx = make_float2(a.x, b.x), ty = make_float2(a.y, b.y);
-  const float2 tz = make_float2(a.z, b.z), tw = make_float2(a.w, b.w);
-  const float2 r24 = make_float2(__uint2float_rn(static_cast<uint32_t>(t0 >> 30) & 0xFFFFFFu),
-                                 __uint2float_rn(static_cast<uint32_t>(t1 >> 30) & 0xFFFFFFu));
-  const float2 d = __fmul2_rn(r24, make_float2(3.657295198167899e-10f, 3.657295198167899e-10f));  // 2*pi / 2^34
-  const float2 d2 = __fmul2_rn(d, d);
-  const float2 nc2 = __fmul2_rn(make_float2(-0.5f, -0.5f), d2);  // cos(d) - 1 (d^4/24 < 6e-11 dropped)
-  const float2 sd = __fmul2_rn(d, __ffma2_rn(d2, make_float2(-0.16666667f, -0.16666667f), make_float2(1.f, 1.f)));
-  const float2 nsd = __fmul2_rn(sd, make_float2(-1.f, -1.f));      // -sin(d)
-  const float2 lr = __ffma2_rn(tx, nc2, __ffma2_rn(tz, nsd, ty));  // z_re - entry_hi
-  const float2 li = __ffma2_rn(tz, nc2, __ffma2_rn(tx, sd, tw));   // z_im - entry_hi
-  two_sum2(tx, lr, zrh, zrl);
-  two_sum2(tz, li, zih, zil);
-}
-
-// Fractional part of x (turns) as a 2^-64 fixed-point value.
-__device__ __forceinline__ uint64_t frac_turns_u64(double x) {
-  const double f = x - rint(x);  // in [-0.5, 0.5]
-  return static_cast<uint64_t>(static_cast<long long>(rint(f * 9223372036854775808.0))) << 1;
-}
-
 // UVWs as (hi, lo) float pairs for the double-float phase set-up.
 static __global__ void split_uvw(const double* __restrict__ uvw, int64_t rows, float* __restrict__ out) {
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < 3 * rows;
@@ -462,117 +395,6 @@ static __global__ void direction_constants(const double* __restrict__ dd, int nd
       out[12 * d + 6 * s + 2 * i + 1] = static_cast<float>(x - static_cast<double>(hi));
     }
   }
-}
-
-// One work item of the compensated reference-antenna pass (batched calls:
-// one per integration chunk).  Blocks are numbered across items.
-struct RefantItem {
-  const float2* vis;       // [C][rows][pols]
-  const double* uvw;       // [rows][3]
-  const double* dd;        // the item's first direction matrix
-  double2* out;            // [nslab][ndir][nI1]
-  int64_t rows;
-  int32_t T, C, pols, ndir;
-  int32_t t_per_slab, c_per_slab, n_tslab, n_cslab;
-  int32_t dgroups, block_begin, pad_[2];
-};
-
-constexpr int kRefantPrefetch = 16;  // channel loads in flight per lane in the compensated pass
-
-// The compensated reference-antenna pass of one call: its work items, the reference
-// baselines, and the number of warp tasks (4 per block of the standalone launch).
-struct RefantParams {
-  const RefantItem* items;
-  const int32_t* I1;
-  double f0, df;
-  int32_t nitems, nbl, nI1, ntasks;
-};
-
-// One warp task of the compensated reference-antenna pass: task w is warp w % 4 of block
-// w / 4 of the standalone launch, i.e. directions j0, j0 + 1 of one group of 4*DPW, for the
-// 32 reference baselines of one tile (one per lane), over one (timestep, channel) slab.
-// tab is the double-float twiddle table in shared memory.  Lanes without a baseline, and
-// warps without a direction, have nothing to do (no warp-collective operations here).
-template <int DPW>
-__device__ __forceinline__ void refant_warp_task(const RefantParams& rp, int task, const float4* tab, int lane) {
-  const RefantItem* items = rp.items;
-  const int blk = task >> 2, warp = task & 3;
-  int ii = 0;
-  while (ii + 1 < rp.nitems && items[ii + 1].block_begin <= blk) ++ii;
-  const RefantItem it = items[ii];
-  constexpr int NW = 4;
-  const int nslab = it.n_tslab * it.n_cslab;
-  const int local = blk - it.block_begin;
-  const int ktile = local / (it.dgroups * nslab);
-  const int dg = (local / nslab) % it.dgroups;
-  const int slab = local % nslab;
-  const int k = ktile * 32 + lane;
-  const int j0 = (dg * NW + warp) * DPW;
-  const int ts = slab / it.n_cslab, cs = slab % it.n_cslab;
-  const int t_lo = ts * it.t_per_slab, t_hi = min(it.T, t_lo + it.t_per_slab);
-  const int c_lo = cs * it.c_per_slab, c_hi = min(it.C, c_lo + it.c_per_slab);
-  const int nI1 = rp.nI1, nbl = rp.nbl;
-  if (j0 >= it.ndir || k >= nI1) return;
-  int b = __ldg(rp.I1 + k);
-  if (b < 0) b += nbl;  // VectorRangeSelect wrap-around (LA/math/cpu/vector.h:97-104)
-  const double kA = rp.f0 / kSpeedOfLight, kB = rp.df / kSpeedOfLight;
-  static_assert(DPW == 2, "the two directions of a warp are the halves of paired instructions");
-  DfAcc2 re{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, im = re;
-  for (int t = t_lo; t < t_hi; ++t) {
-    const int64_t r = static_cast<int64_t>(t) * nbl + b;
-    const double uu = __ldg(it.uvw + 3 * r), vv = __ldg(it.uvw + 3 * r + 1), ww = __ldg(it.uvw + 3 * r + 2);
-    uint64_t pa[DPW], pb[DPW];
-#pragma unroll
-    for (int j = 0; j < DPW; ++j) {
-      const int d = min(j0 + j, it.ndir - 1);
-      const double wrot = __ldg(it.dd + 9 * d + 6) * uu + __ldg(it.dd + 9 * d + 7) * vv + __ldg(it.dd + 9 * d + 8) * ww;
-      const double dw = wrot - ww;
-      pa[j] = frac_turns_u64(-dw * kA);
-      pb[j] = frac_turns_u64(-dw * kB);
-    }
-    const float2* src = it.vis + r * it.pols;
-    const int64_t cstride = static_cast<int64_t>(it.rows) * it.pols;
-    // Blocks of kRefantPrefetch channels: all loads of a block are issued before any use,
-    // so each lane keeps that many scattered 8-byte reads in flight (the rows of the
-    // reference-antenna baselines are spread over the cube).
-    for (int c0 = c_lo; c0 < c_hi; c0 += kRefantPrefetch) {
-      float2 vb[kRefantPrefetch];
-#pragma unroll
-      for (int i = 0; i < kRefantPrefetch; ++i)
-        vb[i] = c0 + i < c_hi ? __ldg(src + static_cast<int64_t>(c0 + i) * cstride) : make_float2(0.f, 0.f);
-#pragma unroll
-      for (int i = 0; i < kRefantPrefetch; ++i) {
-        if (c0 + i >= c_hi) break;
-        const float2 v = vb[i];
-        const float2 vx = make_float2(v.x, v.x), nvx = make_float2(-v.x, -v.x);
-        const float2 vy = make_float2(v.y, v.y), nvy = make_float2(-v.y, -v.y);
-        float2 zrh, zrl, zih, zil;
-        df_twiddle2(pa[0] + static_cast<uint64_t>(c0 + i) * pb[0], pa[1] + static_cast<uint64_t>(c0 + i) * pb[1], tab,
-                    zrh, zrl, zih, zil);
-        df_add_product2(re, vx, nvx, zrh, zrl);  // re += vr zr - vi zi
-        df_add_product2(re, nvy, vy, zih, zil);
-        df_add_product2(im, vx, nvx, zih, zil);  // im += vr zi + vi zr
-        df_add_product2(im, vy, nvy, zrh, zrl);
-      }
-    }
-  }
-  double2* out = it.out + static_cast<int64_t>(slab) * it.ndir * nI1;
-  out[static_cast<int64_t>(j0) * nI1 + k] = make_double2(static_cast<double>(re.s.x) + static_cast<double>(re.c.x),
-                                                         static_cast<double>(im.s.x) + static_cast<double>(im.c.x));
-  if (j0 + 1 < it.ndir)
-    out[static_cast<int64_t>(j0 + 1) * nI1 + k] = make_double2(static_cast<double>(re.s.y) + static_cast<double>(re.c.y),
-                                                               static_cast<double>(im.s.y) + static_cast<double>(im.c.y));
-}
-
-// The pass as its own launch: rp.ntasks / 4 blocks of 4 warps.
-template <int DPW>
-__global__ void __launch_bounds__(128, 5) refant_average_df_items(const RefantParams rp,
-                                                                 const float4* __restrict__ df_tab) {
-  __shared__ float4 tab[kTwiddleSize];
-  for (int i = threadIdx.x; i < kTwiddleSize; i += blockDim.x) tab[i] = __ldg(df_tab + i);
-  __syncthreads();
-  refant_warp_task<DPW>(rp, static_cast<int>(blockIdx.x) * 4 + static_cast<int>(threadIdx.x >> 5), tab,
-                        static_cast<int>(threadIdx.x & 31));
 }
 
 // Sum of slab partials in slab order: avg[i] = sum_s partial[s][i].

@@ -2,6 +2,8 @@
 // kernels), the compensated reference-antenna pass, the solve and the contraction, the
 // batched call with its autotuner and graph replay, and the avgData / UVW getters.
 #include "leap_internal.h"
+#include <functional>
+
 #include "kernels_solve.cuh"
 #include "kernels_mma.cuh"
 #include "kernels_fixed.cuh"
@@ -94,7 +96,7 @@ const unsigned char* grid_table_for(leap_ctx* ctx, int C, float& einv) {
 // integrations with a tensor map): a window pass over the units, then one
 // persistent launch, then the slab reduction where items were split.
 int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double* d_dd, int32_t D, cudaStream_t s,
-                  int& kernels) {
+                  const std::function<int()>& refant, int& kernels) {
   Metadata& md = ctx->md;
   const int32_t nbl = static_cast<int32_t>(md.k.nbaselines);
   const int nquad = (nbl + 3) / 4;
@@ -169,7 +171,7 @@ int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const doubl
       partial_elems += static_cast<int64_t>(it.nslab) * w.ndir * 4 * nbl;
     }
   }
-  if (units == 0) return LEAP_OK;
+  if (units == 0) return refant();
   if (partial_elems) LEAP_CUDA(ctx->partial.ensure(sizeof(double2) * partial_elems), "alloc partial sums");
   for (size_t i = 0; i < items.size(); ++i) {
     GridItem& it = git[i];
@@ -225,6 +227,7 @@ int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const doubl
   es_kernel_poly(kGrTaps, kGrBeta, kGrPolyDeg, &gp.wpoly[0][0]);
   grid_windows<<<static_cast<unsigned>(units), kGrWinThreads, 0, s>>>(gp);
   ++kernels;
+  if (const int rc = refant()) return rc;
   if (!ctx->grid_attr) {
     LEAP_CUDA(cudaFuncSetAttribute(rotate_average_gridded<kGrTaps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    grid_smem_bytes()),
@@ -311,8 +314,9 @@ int ensure_spectrum(leap_ctx* ctx, int channels, cudaStream_t s) {
 }
 
 // Rotate + average of every item into ctx->avg ([D][P][nbl]).
+// refant: launches the reference-antenna pass, where the call has one and the gridded kernel takes the bulk.
 int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double* d_dd, int32_t D, int32_t precision,
-                 int P, cudaStream_t s, int& kernels) {
+                 int P, cudaStream_t s, const std::function<int()>& refant, int& kernels) {
   Metadata& md = ctx->md;
   const int32_t nbl = static_cast<int32_t>(md.k.nbaselines);
   const int tiles = (nbl + 31) / 32;
@@ -330,7 +334,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     if (rc != LEAP_OK) return rc;
   }
 
-  if (uses_gridded(ctx, items, D, precision, P)) return gridded_stage(ctx, items, d_dd, D, s, kernels);
+  if (uses_gridded(ctx, items, D, precision, P)) return gridded_stage(ctx, items, d_dd, D, s, refant, kernels);
   if (all_pipe) {
     // Kernel: the tensor-core one (16 directions per unit) when the autotuner chose it or the
     // option forces it (items of at least 12 directions); else the CUDA-core one with as many tiles
@@ -555,12 +559,12 @@ int refant_reduce(leap_ctx* ctx, cudaStream_t st, int& kernels) {
 // Mixed form: compensated sums of pol 0 of the reference-antenna baselines into
 // ctx->avg_i1 ([D][nI1]), on the aux stream.  complex<float> items go through one
 // item-table launch; complex<double> items keep the FP64 kernel.
-int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double* d_dd, int32_t D, int& kernels) {
+int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double* d_dd, int32_t D, cudaStream_t a,
+                 int& kernels) {
   Metadata& md = ctx->md;
   const int32_t nbl = static_cast<int32_t>(md.k.nbaselines);
   const int nI1 = md.A1rows - 1;
   const int rtiles = (nI1 + 31) / 32;
-  cudaStream_t a = ctx->aux;
   LEAP_CUDA(ctx->avg_i1.ensure(sizeof(double2) * static_cast<int64_t>(D) * nI1), "alloc I1 sums");
   std::vector<RefantItem>& rit = ctx->refant_items_host;
   std::vector<ReduceItem>& red = ctx->refant_reduce_host;
@@ -569,18 +573,22 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
   int64_t partial_elems = 0;
   std::vector<int64_t> off;
   int blocks = 0;
-  // Each block sums 4*DPW directions of 32 reference baselines over a slab of
-  // (timestep, channel) pairs.  Slabs are sized to one budget across items (about
-  // 10 blocks per SM in total, two waves of the 5 resident blocks), so that chunks
-  // of 1 x 48 and 64 x 384 samples give blocks of similar length instead of the same
-  // number of blocks each; fewer, longer slabs also keep the partial sums (and their
-  // reduction) small.
-  int64_t work_total = 0;
+  // Each block sums kRefWarps directions of 32 reference baselines over a slab of (timestep, channel) pairs.  Slabs of
+  // whole timesteps are sized to one budget across items (about 12 blocks per SM in total, four waves of the 3
+  // resident blocks), so that chunks of 1 x 48 and 64 x 384 samples give blocks of similar length; fewer, longer
+  // slabs also keep the partial sums (and their reduction) small.  The phasors of a row's 16 channel offsets are formed
+  // per slab, so channels are split only where timesteps alone leave SMs without two blocks, and in whole rounds.
+  int64_t work_total = 0, t_blocks = 0;
   for (const auto& w : items) {
     const Integration& in = ctx->integ.at(w.slot);
-    work_total += (in.rows / nbl) * in.channels * rtiles * ((w.ndir + 7) / 8);
+    if (in.vis_type != LEAP_VIS_C64) continue;
+    const int64_t tiles = static_cast<int64_t>(rtiles) * ((w.ndir + kRefWarps - 1) / kRefWarps);
+    work_total += (in.rows / nbl) * in.channels * tiles;
+    t_blocks += (in.rows / nbl) * tiles;
   }
-  const int64_t slab_budget = std::max<int64_t>(64, (work_total + 10 * ctx->sms - 1) / (10 * ctx->sms));
+  const int64_t slab_budget = std::max<int64_t>(64, (work_total + 12 * ctx->sms - 1) / (12 * ctx->sms));
+  const int64_t c_split =
+      t_blocks > 0 && t_blocks < 2 * ctx->sms ? (3 * ctx->sms + t_blocks - 1) / t_blocks : 1;
   for (const auto& w : items) {
     Integration& in = ctx->integ.at(w.slot);
     const int T = static_cast<int>(in.rows / nbl);
@@ -630,16 +638,15 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     r.C = in.channels;
     r.pols = in.pols;
     r.ndir = w.ndir;
-    r.dgroups = (w.ndir + 7) / 8;  // 4 warps x 2 directions
+    r.dgroups = (w.ndir + kRefWarps - 1) / kRefWarps;
     const int64_t want =
         std::max<int64_t>(1, (static_cast<int64_t>(T) * in.channels + slab_budget - 1) / slab_budget);
     r.n_tslab = static_cast<int>(std::min<int64_t>(T, want));
     r.t_per_slab = (T + r.n_tslab - 1) / r.n_tslab;
     r.n_tslab = (T + r.t_per_slab - 1) / r.t_per_slab;
-    const int64_t rest = (want + r.n_tslab - 1) / r.n_tslab;
-    r.n_cslab = static_cast<int>(std::min<int64_t>(rest, std::max(1, in.channels / 16)));
-    r.c_per_slab = (in.channels + r.n_cslab - 1) / r.n_cslab;
-    if (r.n_cslab > 1) r.c_per_slab = (r.c_per_slab + 15) / 16 * 16;  // whole blocks of kRefantPrefetch loads
+    const int rounds = (in.channels + kRefRound - 1) / kRefRound;
+    const int n_cslab = static_cast<int>(std::min<int64_t>(c_split, rounds));
+    r.c_per_slab = (rounds + n_cslab - 1) / n_cslab * kRefRound;
     r.n_cslab = (in.channels + r.c_per_slab - 1) / r.c_per_slab;
     r.block_begin = blocks;
     blocks += rtiles * r.dgroups * r.n_tslab * r.n_cslab;
@@ -672,10 +679,19 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
   rp.nitems = static_cast<int32_t>(rit.size());
   rp.nbl = nbl;
   rp.nI1 = nI1;
-  rp.ntasks = blocks * 4;
-  refant_average_df_items<2><<<blocks, 128, 0, a>>>(rp, ctx->twiddle_df.as<float4>());
+  if (!ctx->refant_attr_set) {
+    LEAP_CUDA(cudaFuncSetAttribute(refant_average_items, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   refant_smem_bytes()),
+              "refant shared memory");
+    ctx->refant_attr_set = true;
+  }
+  refant_average_items<<<blocks, kRefWarps * 32, refant_smem_bytes(), a>>>(rp, ctx->twiddle_df.as<float4>());
   ++kernels;
-  return refant_reduce(ctx, a, kernels);
+  if (a != ctx->aux) {  // the sums of the slabs beside what the stream does next
+    LEAP_CUDA(cudaEventRecord(ctx->fork, a), "fork");
+    LEAP_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->fork, 0), "fork");
+  }
+  return refant_reduce(ctx, ctx->aux, kernels);
 }
 
 template <int N>
@@ -810,28 +826,30 @@ int calibrate_items(leap_ctx* ctx, const std::vector<WorkItem>& items, const dou
   cudaEvent_t* ev = ctx->ring[ctx->ring_count % leap_ctx::kRing];
   if (!ctx->capturing) cudaEventRecord(ev[0], s);
   const bool refant = precision == LEAP_PRECISION_MIXED && md.A1rows > 1;
-  if (refant) {
+  const bool gridded = uses_gridded(ctx, items, D, precision, P);
+  if (refant && !gridded) {
     LEAP_CUDA(cudaEventRecord(ctx->fork, s), "fork");
     LEAP_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->fork, 0), "fork");
   }
   // The reference-antenna pass cannot share an SM with either bulk kernel (registers or shared
   // memory; running it on extra warps of the gridded kernel measured slower than two launches).
-  // Beside the gridded kernel it goes first, so that it overlaps the small kernels that set up
-  // the grid windows; beside the pipelined kernel it goes after it, so that the persistent
-  // blocks, whose unit schedule assumes they start together, take the SMs first.
-  const bool refant_first = refant && uses_gridded(ctx, items, D, precision, P);
-  int rc = LEAP_OK;
-  if (refant_first) {
-    rc = refant_stage(ctx, items, d_dd, D, kernels);
+  // Before the gridded kernel it takes its turn on the call's stream, after the kernels that set up the grid windows:
+  // beside them it kept them waiting (its blocks stay on their SMs for all of its time; 128 antennas, 64 directions:
+  // 667 us a call, 658 in turn), and gridded blocks that start while it runs are late where it took their SM (730
+  // us).  Beside the pipelined kernel it goes second, so that the persistent blocks, whose unit schedule assumes they
+  // start together, take the SMs first.
+  auto pass = [&]() -> int {
+    if (!refant) return LEAP_OK;
+    const int rc = refant_stage(ctx, items, d_dd, D, gridded ? s : ctx->aux, kernels);
     if (rc != LEAP_OK) return rc;
     LEAP_CUDA(cudaEventRecord(ctx->join, ctx->aux), "join");
-  }
-  rc = rotate_stage(ctx, items, d_dd, D, precision, P, s, kernels);
+    return LEAP_OK;
+  };
+  int rc = rotate_stage(ctx, items, d_dd, D, precision, P, s, pass, kernels);
   if (rc != LEAP_OK) return rc;
-  if (refant && !refant_first) {
-    rc = refant_stage(ctx, items, d_dd, D, kernels);
+  if (!gridded) {
+    rc = pass();
     if (rc != LEAP_OK) return rc;
-    LEAP_CUDA(cudaEventRecord(ctx->join, ctx->aux), "join");
   }
   if (!ctx->capturing) cudaEventRecord(ev[1], s);
   if (refant) LEAP_CUDA(cudaStreamWaitEvent(s, ctx->join, 0), "join");

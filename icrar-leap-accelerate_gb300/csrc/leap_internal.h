@@ -21,6 +21,7 @@
 #include "leap_gb300.h"
 #include "host_math.h"
 #include "kernels_rotate.cuh"
+#include "kernels_refant.cuh"
 #include "kernels_grid.cuh"
 
 
@@ -133,6 +134,7 @@ struct leap_ctx {
   std::vector<int32_t> grid_order_host;
   DeviceBuffer grid_items, grid_order, grid_win;
   bool pipe_attr_mma = false;
+  bool refant_attr_set = false;       // its shared-memory size was raised
   int tc_attr_set = 0;                // bit per N tile whose shared-memory size was raised
   DeviceBuffer dphi_tc;               // packed dphi operand of the tensor-core contraction
   DeviceBuffer adj_dphi, adj_cal1, adj_phi1, adj_gavg, adj_partial, adj_g, adj_gexp;  // adjoint scratch
