@@ -538,7 +538,34 @@ static __global__ void adjoint_contract_t(const double* __restrict__ M, int S, i
   const int lane = threadIdx.x & 31;
   if (k >= kmax) return;
   const double* col = M + static_cast<int64_t>(S) * k;
-  for (int d = 0; d < D; ++d) {
+  // 16 directions at a time are summed over the lanes together, halving the directions that a lane holds with each
+  // exchange: 16 additions instead of 80, which with the 64 products (128 stations) are bound by the FP64 pipe (128
+  // stations, 16 directions, 8128 rows: 73 -> 48 us).  Up to 3 directions, fewer additions one by one.
+  int d_lo = 0;
+  for (; D - d_lo > 3; d_lo += 16) {
+    double x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = 0.0;
+    for (int s = lane; s < S; s += 32) {
+      const double c = col[s];
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (d_lo + i < D) x[i] += c * G[static_cast<int64_t>(d_lo + i) * S + s];
+    }
+#pragma unroll
+    for (int n = 8; n > 0; n >>= 1) {
+      const bool up = lane & (2 * n);
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const double y = __shfl_xor_sync(0xffffffffu, up ? x[i] : x[i + n], 2 * n);
+        x[i] = (up ? x[i + n] : x[i]) + y;
+      }
+    }
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+    const int d = d_lo + (lane >> 1);
+    if (!(lane & 1) && d < D) out[static_cast<int64_t>(d) * ldo + k] = x[0];
+  }
+  for (int d = d_lo; d < D; ++d) {
     double x = 0.0;
     for (int s = lane; s < S; s += 32) x += col[s] * G[static_cast<int64_t>(d) * S + s];
 #pragma unroll

@@ -118,7 +118,10 @@ static __global__ void solve_dint_mixed(SolveArgs a) {
 }
 
 // K6: partial[kc][d][s] = sum_{k in chunk kc} Ad[s, k] * dphi[d][k].
-// Block tile: 64 stations x 16 directions, 256 threads, 4 outputs per thread.
+// Block tile: 64 stations x 16 directions, 256 threads, 4 outputs per thread.  In FP64 a block's 512 x 64 x 16 products
+// take 137 us of its SM's FP64 pipe (2 lanes per clock), so chunks are cut until there are two blocks per SM
+// (contraction_chunk), and warps without a direction, and directions past the last, compute nothing.  36 antennas and
+// one direction: 169 -> 7 us; 128 antennas, 64 directions: 177 -> 135 us (116 us of products over all SMs).
 template <typename T>
 static __global__ void __launch_bounds__(256) gemm_ad_partial(const T* __restrict__ Ad, int S, int Arows,
                                                        const T* __restrict__ dphi, int Kpad, int ndir,
@@ -130,6 +133,7 @@ static __global__ void __launch_bounds__(256) gemm_ad_partial(const T* __restric
   const int k_begin = kc * kchunk, k_end = min(Arows, k_begin + kchunk);
   const int tx = threadIdx.x & 63;   // station within tile
   const int ty = threadIdx.x >> 6;   // 0..3 -> directions ty, ty+4, ty+8, ty+12
+  const int nq = max(0, min(4, (ndir - d0 - ty + 3) >> 2));  // directions of this warp
   T acc[4] = {T(0), T(0), T(0), T(0)};
   for (int k0 = k_begin; k0 < k_end; k0 += TK) {
     for (int i = threadIdx.x; i < TK * TS; i += 256) {
@@ -143,11 +147,20 @@ static __global__ void __launch_bounds__(256) gemm_ad_partial(const T* __restric
       sB[dd][kk] = (k < k_end && d < ndir) ? dphi[static_cast<int64_t>(d) * Kpad + k] : T(0);
     }
     __syncthreads();
+    if (nq == 4) {
 #pragma unroll 8
-    for (int kk = 0; kk < TK; ++kk) {
-      const T av = sA[kk][tx];
+      for (int kk = 0; kk < TK; ++kk) {
+        const T av = sA[kk][tx];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] += av * sB[ty + 4 * q][kk];
+        for (int q = 0; q < 4; ++q) acc[q] += av * sB[ty + 4 * q][kk];
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (q < nq) {
+#pragma unroll 8
+          for (int kk = 0; kk < TK; ++kk) acc[q] += sA[kk][tx] * sB[ty + 4 * q][kk];
+        }
     }
     __syncthreads();
   }

@@ -738,12 +738,21 @@ int tc_contraction(leap_ctx* ctx, int32_t D, double* d_cal, cudaStream_t s, int&
   return LEAP_OK;
 }
 
+// Rows of A per block of the direct contraction (gemm_ad_partial): as many as leave two blocks per SM, in steps of its
+// stages of 32; at most 512, so that a large one's partial sums stay few.
+int contraction_chunk(const leap_ctx* ctx, int D) {
+  const int tiles = ((ctx->md.S + 63) / 64) * ((D + 15) / 16);
+  const int want = std::max(1, 2 * ctx->sms / tiles);
+  const int rows = (ctx->md.Arows + want - 1) / want;
+  return std::min(512, std::max(32, (rows + 31) / 32 * 32));
+}
+
 // Phase angles + both contractions for all D directions: avg -> cal.
 int solve_stage(leap_ctx* ctx, int32_t D, int32_t precision, int P, bool refant, double* d_cal, cudaStream_t s,
                 int& kernels) {
   Metadata& md = ctx->md;
   const int32_t nbl = static_cast<int32_t>(md.k.nbaselines);
-  const int kchunk = 512;
+  const int kchunk = contraction_chunk(ctx, D);
   const int nk = (md.Arows + kchunk - 1) / kchunk;
   SolveArgs sa{};
   sa.avg = ctx->avg.as<double2>();
@@ -813,7 +822,7 @@ int calibrate_items(leap_ctx* ctx, const std::vector<WorkItem>& items, const dou
     P = it->second.pols;
   }
   const int64_t avg_elems = static_cast<int64_t>(D) * P * nbl;
-  const int kchunk = 512;
+  const int kchunk = contraction_chunk(ctx, D);
   const int nk = (md.Arows + kchunk - 1) / kchunk;
   LEAP_CUDA(ctx->avg.ensure(sizeof(double2) * avg_elems), "alloc avgData");
   LEAP_CUDA(ctx->dirk.ensure(sizeof(float) * 12 * D), "alloc direction constants");
