@@ -19,6 +19,7 @@
 #pragma once
 
 #include "leap_common.cuh"
+#include "narrow.h"
 #include "kernels_pipe.cuh"
 
 namespace leapgb {
@@ -49,13 +50,6 @@ __device__ __forceinline__ void load_sample(const VisT* __restrict__ p, double& 
   const VisT v = __ldg(p);
   re = static_cast<double>(v.x);
   im = static_cast<double>(v.y);
-}
-
-template <typename VisT>
-__device__ __forceinline__ void load_sample_f(const VisT* __restrict__ p, float& re, float& im) {
-  const VisT v = __ldg(p);
-  re = static_cast<float>(v.x);
-  im = static_cast<float>(v.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -193,11 +187,18 @@ __global__ void __launch_bounds__(128) rotate_average_fp64(RotateArgs a) {
 // sums) and FP32 complex MACs.
 // Sums run in FP32 over blocks of KB channels and are folded into Kahan
 // (sum, compensation) pairs, written out as sum - compensation in FP64.
+//
+// Bound by latency (the loads' and the table's) and by the issue slots: 7 blocks per SM (72 registers) and the loads of
+// one or two groups of samples ahead do better than more of either; complex<double> samples are converted on the
+// integer pipe (narrow.h).  128 antennas, 4 timesteps, 96 channels, 16 directions, two complex<double> pols: a call
+// 365 -> 231 us with the FP64 pass over the reference baselines above (4 or 8 samples ahead: 282 and 333; 8 or 10
+// blocks: 231 and 245; converted by the conversion instruction: 269).
 // ---------------------------------------------------------------------------
 template <typename VisT, int P, int DPW>
-__global__ void __launch_bounds__(128) rotate_average_mixed(RotateArgs a) {
+__global__ void __launch_bounds__(128, P == 4 ? 4 : 7) rotate_average_mixed(RotateArgs a) {
   constexpr int NW = 4;
   constexpr int KB = 16;
+  constexpr int KU = 4 / P;  // channels whose loads are on their way together
   __shared__ float2 tab[kTwiddleSize];
   for (int i = threadIdx.x; i < kTwiddleSize; i += blockDim.x) tab[i] = __ldg(a.twiddle + i);
   __syncthreads();
@@ -240,19 +241,32 @@ __global__ void __launch_bounds__(128) rotate_average_mixed(RotateArgs a) {
         for (int j = 0; j < DPW; ++j)
 #pragma unroll
           for (int p = 0; p < P; ++p) pr[j][p] = pi[j][p] = 0.f;
-        for (int c = cb; c < ce; ++c) {
-          const VisT* src = vis + (static_cast<int64_t>(c) * a.rows + r) * P;
-          float vr[P], vi[P];
+        for (int c0 = cb; c0 < ce; c0 += KU) {
+          VisT raw[KU][P];
 #pragma unroll
-          for (int p = 0; p < P; ++p) load_sample_f(src + p, vr[p], vi[p]);
+          for (int k = 0; k < KU; ++k)
 #pragma unroll
-          for (int j = 0; j < DPW; ++j) {
-            float s, co;
-            twiddle_turns(pa[j] + static_cast<uint32_t>(c) * pb[j], tab, co, s);
+            for (int p = 0; p < P; ++p)
+              raw[k][p] = __ldg(vis + (static_cast<int64_t>(min(c0 + k, ce - 1)) * a.rows + r) * P + p);
+#pragma unroll
+          for (int k = 0; k < KU; ++k) {
+            const int c = c0 + k;
+            if (c >= ce) break;
+            float vr[P], vi[P];
 #pragma unroll
             for (int p = 0; p < P; ++p) {
-              pr[j][p] = fmaf(vr[p], co, fmaf(-vi[p], s, pr[j][p]));
-              pi[j][p] = fmaf(vr[p], s, fmaf(vi[p], co, pi[j][p]));
+              vr[p] = narrow(raw[k][p].x);
+              vi[p] = narrow(raw[k][p].y);
+            }
+#pragma unroll
+            for (int j = 0; j < DPW; ++j) {
+              float s, co;
+              twiddle_turns(pa[j] + static_cast<uint32_t>(c) * pb[j], tab, co, s);
+#pragma unroll
+              for (int p = 0; p < P; ++p) {
+                pr[j][p] = fmaf(vr[p], co, fmaf(-vi[p], s, pr[j][p]));
+                pi[j][p] = fmaf(vr[p], s, fmaf(vi[p], co, pi[j][p]));
+              }
             }
           }
         }
@@ -297,6 +311,8 @@ __global__ void __launch_bounds__(128) rotate_average_mixed(RotateArgs a) {
 // rotate_average_fp64, pol 0 only), gathered by I1.  They are 1-2% of the rows
 // and use the FP64 pipe, which the FP32 bulk kernel leaves idle, so the call
 // launches this kernel on a second stream to overlap the two.
+// (128 antennas, 4 timesteps, 96 channels, 16 directions, alone: 70 -> 35 us with Horner's rule, and slabs of 16 channels
+// where longer ones leave SMs without a block.)
 // Output: [nslab][ndir][nI1] double2 (nslab == 1: final).
 // ---------------------------------------------------------------------------
 template <typename VisT, int DPW>
@@ -341,20 +357,29 @@ __global__ void __launch_bounds__(128) refant_average_fp64(RotateArgs a, const i
     }
     for (int cb = c_lo; cb < c_hi; cb += kSeed) {
       const int ce = min(c_hi, cb + kSeed);
-      double zr[DPW], zi[DPW];
+      // Horner's rule in the step's phasor from the block's last channel on, then the first channel's phasor: four FMAs
+      // per channel and direction instead of the eight that advance a phasor and add its product.
+      double hr[DPW], hi[DPW];
 #pragma unroll
-      for (int j = 0; j < DPW; ++j) sincos(sf[j] / __ldg(a.lambda + cb), &zi[j], &zr[j]);
-      for (int c = cb; c < ce; ++c) {
+      for (int j = 0; j < DPW; ++j) hr[j] = hi[j] = 0.0;
+      const VisT* src = vis + (static_cast<int64_t>(cb) * a.rows + r) * a.pols;
+#pragma unroll 8
+      for (int c = ce - cb - 1; c >= 0; --c) {
         double vr, vi;
-        load_sample(vis + (static_cast<int64_t>(c) * a.rows + r) * a.pols, vr, vi);
+        load_sample(src + c * a.rows * a.pols, vr, vi);
 #pragma unroll
         for (int j = 0; j < DPW; ++j) {
-          accr[j] += vr * zr[j] - vi * zi[j];
-          acci[j] += vr * zi[j] + vi * zr[j];
-          const double nr = zr[j] * wr[j] - zi[j] * wi[j];
-          zi[j] = zr[j] * wi[j] + zi[j] * wr[j];
-          zr[j] = nr;
+          const double nr = fma(-hi[j], wi[j], fma(hr[j], wr[j], vr));
+          hi[j] = fma(hi[j], wr[j], fma(hr[j], wi[j], vi));
+          hr[j] = nr;
         }
+      }
+#pragma unroll
+      for (int j = 0; j < DPW; ++j) {
+        double zr, zi;
+        sincos(sf[j] / __ldg(a.lambda + cb), &zi, &zr);
+        accr[j] += hr[j] * zr - hi[j] * zi;
+        acci[j] += hr[j] * zi + hi[j] * zr;
       }
     }
   }

@@ -596,7 +596,7 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
       // FP64 kernel for complex<double> input, one launch per item.
       int rt_per, rc_per, rnts, rncs;
       const int rdg = (w.ndir + 7) / 8;
-      choose_slabs_target(T, in.channels, static_cast<int64_t>(rtiles) * rdg, ctx->sms, rt_per, rc_per, rnts, rncs);
+      choose_slabs_target(T, in.channels, static_cast<int64_t>(rtiles) * rdg, 2 * ctx->sms, rt_per, rc_per, rnts, rncs, 16);
       const int rslab = rnts * rncs;
       const int64_t n = static_cast<int64_t>(w.ndir) * nI1;
       LEAP_CUDA(ctx->partial_i1.ensure(sizeof(double2) * n * rslab), "alloc I1 partials");

@@ -228,10 +228,10 @@ inline int grid_1d(int64_t n, int threads) {
 
 // Slab split of (timestep, channel) space so that the grid reaches `target` blocks.
 inline void choose_slabs_target(int timesteps, int channels, int64_t base_blocks, int64_t target, int& t_per, int& c_per,
-                         int& nts, int& ncs) {
+                         int& nts, int& ncs, int min_pairs = 64) {
   int64_t want = std::max<int64_t>(1, (target + base_blocks - 1) / base_blocks);
-  // Keep at least 64 (timestep, channel) pairs per slab.
-  const int64_t max_slabs = std::max<int64_t>(1, (static_cast<int64_t>(timesteps) * channels) / 64);
+  // Keep at least min_pairs (timestep, channel) pairs per slab.
+  const int64_t max_slabs = std::max<int64_t>(1, (static_cast<int64_t>(timesteps) * channels) / min_pairs);
   want = std::min(want, max_slabs);
   nts = static_cast<int>(std::min<int64_t>(want, timesteps));
   t_per = (timesteps + nts - 1) / nts;
