@@ -249,12 +249,14 @@ inline void choose_slabs(int timesteps, int channels, int64_t base_blocks, int& 
 
 // Slab split for the fixed-point kernel, `resident` of whose blocks run at a time: the fewest slabs whose
 // blocks fill the last round of resident ones to 95%, of whole timesteps, then of 128-channel sums, and of
-// 32-channel blocks (the seeding interval) only where the call is too small to fill the GPU once.
+// 32-channel blocks (the seeding interval) or 16-channel ones (a stage) only where the call is too small to fill the
+// GPU once (36 antennas, 48 channels, one direction: 145 us a call in 32s, 104 in 16s; in 8s 97, but another small call
+// 8% slower).
 inline void choose_fixed_slabs(int timesteps, int channels, int64_t base_blocks, int64_t resident, int& t_per, int& c_per,
                                int& nts, int& ncs) {
   double best_eff = -1.0;
   t_per = timesteps; c_per = channels; nts = ncs = 1;
-  for (int unit : {128, 32}) {
+  for (int unit : {128, 32, 16}) {
     const int max_c = (channels + unit - 1) / unit;
     for (int c = 1; c <= max_c; ++c) {
       const int cp = ((channels + c - 1) / c + unit - 1) / unit * unit;
