@@ -215,9 +215,11 @@ struct DeviceGuard {
 };
 
 constexpr int kPipeNC = 8;   // warps of the pipelined kernel
-// Directions per item from which the gridded kernel is the default: its grid product costs
-// about as much as ~25 directions of the pipelined kernel's per-direction work (measured on
-// 128 antennas x 384 channels: 64 directions 1.29 vs 2.86 ms; 8 per item 35 vs 14 ms).
+// Directions per item from which the gridded kernel is the default.  128 antennas, 14 timesteps, 384 channels near the
+// phase centre, pipelined against gridded: 32 directions 1217 and 547 us a call, 24 1191 and 490, 16 695 and 468.  The line
+// is not lower because a new integration's operand adds 510 us to its first gridded call, and because directions far
+// from the phase centre need several grid passes (nine of them: 0.58 and 1.68 ms).  Small calls would be better off
+// pipelined (64 antennas, 8 timesteps, 128 channels, 32 directions: 180 and 202 us), at a larger error.
 constexpr int kGridAutoDirs = 32;
 constexpr int kPipeDPW = 4;  // directions per warp
 
