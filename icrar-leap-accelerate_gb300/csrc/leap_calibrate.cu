@@ -574,9 +574,10 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
   std::vector<int64_t> off;
   int blocks = 0;
   // Each block sums kRefWarps directions of 32 reference baselines over a slab of (timestep, channel) pairs.  Slabs of
-  // whole timesteps are sized to one budget across items (about 12 blocks per SM in total, four waves of the 3
+  // whole timesteps are sized to one budget across items (about 24 blocks per SM in total, eight waves of the 3
   // resident blocks), so that chunks of 1 x 48 and 64 x 384 samples give blocks of similar length; fewer, longer
-  // slabs also keep the partial sums (and their reduction) small.  The phasors of a row's 16 channel offsets are formed
+  // slabs keep the partial sums (and their reduction) small, but leave a longer last wave (131328 rows, 128 directions:
+  // 15.84 ms a call with 12 blocks per SM, 15.61 with 24; the 52 GB batch 10.38 and 10.39).  The phasors of a row's 16 channel offsets are formed
   // per slab, so channels are split only where timesteps alone leave SMs without two blocks, and in whole rounds.
   int64_t work_total = 0, t_blocks = 0;
   for (const auto& w : items) {
@@ -586,7 +587,7 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     work_total += (in.rows / nbl) * in.channels * tiles;
     t_blocks += (in.rows / nbl) * tiles;
   }
-  const int64_t slab_budget = std::max<int64_t>(64, (work_total + 12 * ctx->sms - 1) / (12 * ctx->sms));
+  const int64_t slab_budget = std::max<int64_t>(64, (work_total + 24 * ctx->sms - 1) / (24 * ctx->sms));
   const int64_t c_split =
       t_blocks > 0 && t_blocks < 2 * ctx->sms ? (3 * ctx->sms + t_blocks - 1) / t_blocks : 1;
   for (const auto& w : items) {
