@@ -92,6 +92,26 @@ const unsigned char* grid_table_for(leap_ctx* ctx, int C, float& einv) {
   return b.as<unsigned char>();
 }
 
+// The split grid operand of an integration and its scales: built once per upload (the visibilities read twice, hi and
+// lo written), then read by every gridded call on it.
+int ensure_grid_operand(leap_ctx* ctx, Integration& in, cudaStream_t s, int& kernels) {
+  const int32_t nbl = static_cast<int32_t>(ctx->md.k.nbaselines);
+  if (in.op_nbl == nbl) return LEAP_OK;
+  if (ctx->capturing) return fail(ctx, LEAP_ERR_INTERNAL, "grid operand missing while recording a graph");
+  in.op_nbl = 0;
+  const int T = static_cast<int>(in.rows / nbl), C = in.channels;
+  const int64_t op_bytes = grid_operand_bytes(nbl, T, C);
+  LEAP_CUDA(in.op.ensure(static_cast<size_t>(op_bytes + grid_scale_bytes(nbl, T))), "alloc grid operand");
+  const dim3 og((nbl + 3) / 4, (T + 3) / 4);
+  grid_split_operand<<<og, kGrSplitThreads, 0, s>>>(in.vis.as<float>(), in.rows, nbl, T, C, (T + 3) / 4,
+                                                    in.op.as<unsigned char>(),
+                                                    reinterpret_cast<float*>(in.op.as<unsigned char>() + op_bytes));
+  LEAP_CUDA(cudaGetLastError(), "grid operand launch");
+  ++kernels;
+  in.op_nbl = nbl;
+  return LEAP_OK;
+}
+
 // Rotate + average of every item through the gridded kernel (4-pol complex<float>
 // integrations with a tensor map): a window pass over the units, then one
 // persistent launch, then the slab reduction where items were split.
@@ -123,19 +143,7 @@ int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const doubl
     const int T = static_cast<int>(in.rows / nbl);
     const int C = in.channels;
     const int64_t op_bytes = grid_operand_bytes(nbl, T, C);
-    if (in.op_nbl != nbl) {
-      // The split grid operand and its scales: built once per upload (the visibilities read
-      // twice, hi and lo written), then read by every gridded call on this integration.
-      if (ctx->capturing) return fail(ctx, LEAP_ERR_INTERNAL, "grid operand missing while recording a graph");
-      LEAP_CUDA(in.op.ensure(static_cast<size_t>(op_bytes + grid_scale_bytes(nbl, T))), "alloc grid operand");
-      const dim3 og((nbl + 3) / 4, (T + 3) / 4);
-      grid_split_operand<<<og, kGrSplitThreads, 0, s>>>(in.vis.as<float>(), in.rows, nbl, T, C, (T + 3) / 4,
-                                            in.op.as<unsigned char>(),
-                                            reinterpret_cast<float*>(in.op.as<unsigned char>() + op_bytes));
-      LEAP_CUDA(cudaGetLastError(), "grid operand launch");
-      ++kernels;
-      in.op_nbl = nbl;
-    }
+    if (const int rc = ensure_grid_operand(ctx, in, s, kernels)) return rc;
     float einv = 1.f;
     const unsigned char* tab = grid_table_for(ctx, C, einv);
     if (!tab) return fail(ctx, LEAP_ERR_CUDA, "grid matrix unavailable for this channel count");
@@ -193,20 +201,20 @@ int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const doubl
       });
     std::vector<int32_t>& order = ctx->grid_order_host;
     schedule_units(std::move(runs), grid, order);
-    LEAP_CUDA(ctx->grid_order.ensure(sizeof(int32_t) * order.size()), "alloc unit order");
+    LEAP_CUDA(ctx->tab->grid_order.ensure(sizeof(int32_t) * order.size()), "alloc unit order");
     if (!ctx->capturing)
-      LEAP_CUDA(cudaMemcpyAsync(ctx->grid_order.ptr, order.data(), sizeof(int32_t) * order.size(),
+      LEAP_CUDA(cudaMemcpyAsync(ctx->tab->grid_order.ptr, order.data(), sizeof(int32_t) * order.size(),
                                 cudaMemcpyHostToDevice, s),
                 "upload unit order");
   }
-  LEAP_CUDA(ctx->grid_items.ensure(sizeof(GridItem) * git.size()), "alloc item table");
+  LEAP_CUDA(ctx->tab->grid_items.ensure(sizeof(GridItem) * git.size()), "alloc item table");
   LEAP_CUDA(ctx->grid_win.ensure(sizeof(GridWindow) * units), "alloc grid windows");
   if (!ctx->capturing)
-    LEAP_CUDA(cudaMemcpyAsync(ctx->grid_items.ptr, git.data(), sizeof(GridItem) * git.size(), cudaMemcpyHostToDevice, s),
+    LEAP_CUDA(cudaMemcpyAsync(ctx->tab->grid_items.ptr, git.data(), sizeof(GridItem) * git.size(), cudaMemcpyHostToDevice, s),
               "upload item table");
   if (!red.empty() && !ctx->capturing) {
-    LEAP_CUDA(ctx->reduce_items.ensure(sizeof(ReduceItem) * red.size()), "alloc reduce table");
-    LEAP_CUDA(cudaMemcpyAsync(ctx->reduce_items.ptr, red.data(), sizeof(ReduceItem) * red.size(),
+    LEAP_CUDA(ctx->tab->reduce_items.ensure(sizeof(ReduceItem) * red.size()), "alloc reduce table");
+    LEAP_CUDA(cudaMemcpyAsync(ctx->tab->reduce_items.ptr, red.data(), sizeof(ReduceItem) * red.size(),
                               cudaMemcpyHostToDevice, s),
               "upload reduce table");
   }
@@ -214,8 +222,8 @@ int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const doubl
                                                    ctx->dirk.as<float>());
   ++kernels;
   GridParams gp{};
-  gp.items = ctx->grid_items.as<GridItem>();
-  gp.order = ctx->grid_order.as<int32_t>();
+  gp.items = ctx->tab->grid_items.as<GridItem>();
+  gp.order = ctx->tab->grid_order.as<int32_t>();
   gp.win = ctx->grid_win.as<GridWindow>();
   gp.dirk = ctx->dirk.as<float>();
   gp.twiddle = ctx->twiddle.as<float2>();
@@ -240,7 +248,7 @@ int gridded_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const doubl
     int64_t maxn = 0;
     for (const auto& r : red) maxn = std::max<int64_t>(maxn, static_cast<int64_t>(r.ndir) * 4 * nbl);
     const dim3 rg(static_cast<unsigned>(std::min<int64_t>((maxn + 255) / 256, 1024)), static_cast<unsigned>(red.size()));
-    reduce_item_slabs<<<rg, 256, 0, s>>>(ctx->reduce_items.as<ReduceItem>(), static_cast<int>(red.size()), 4 * nbl,
+    reduce_item_slabs<<<rg, 256, 0, s>>>(ctx->tab->reduce_items.as<ReduceItem>(), static_cast<int>(red.size()), 4 * nbl,
                                           ctx->avg.as<double2>());
     ++kernels;
   }
@@ -283,29 +291,29 @@ int launch_pipe(leap_ctx* ctx, const PipeParams& pp, int grid, cudaStream_t s) {
 // the fixed-point spectral window; uploaded only when the channel count or the spectral window changes.
 int ensure_spectrum(leap_ctx* ctx, int channels, cudaStream_t s) {
   const Metadata& md = ctx->md;
-  LEAP_CUDA(ctx->lambda.ensure(sizeof(double) * 2 * channels), "alloc wavelengths");
-  if (ctx->lambda_host.size() != static_cast<size_t>(2 * channels) || ctx->lambda_f0 != md.k.freq_start_hz ||
-      ctx->lambda_df != md.k.freq_inc_hz) {
+  LEAP_CUDA(ctx->tab->lambda.ensure(sizeof(double) * 2 * channels), "alloc wavelengths");
+  if (ctx->tab->lambda_host.size() != static_cast<size_t>(2 * channels) || ctx->tab->lambda_f0 != md.k.freq_start_hz ||
+      ctx->tab->lambda_df != md.k.freq_inc_hz) {
     // [wavelengths][their reciprocals]: c / (f0 + ch*df) with each operation rounded on its own,
     // as the reference's Constants::GetChannelWavelength (no fused multiply-add).
-    ctx->lambda_host.resize(2 * channels);
+    ctx->tab->lambda_host.resize(2 * channels);
     for (int c = 0; c < channels; ++c) {
       volatile double prod = static_cast<double>(c) * md.k.freq_inc_hz;
       const double lam = kSpeedOfLight / (md.k.freq_start_hz + prod);
-      ctx->lambda_host[c] = lam;
-      ctx->lambda_host[channels + c] = 1.0 / lam;
+      ctx->tab->lambda_host[c] = lam;
+      ctx->tab->lambda_host[channels + c] = 1.0 / lam;
     }
-    ctx->lambda_f0 = md.k.freq_start_hz;
-    ctx->lambda_df = md.k.freq_inc_hz;
-    LEAP_CUDA(cudaMemcpyAsync(ctx->lambda.ptr, ctx->lambda_host.data(), sizeof(double) * 2 * channels,
+    ctx->tab->lambda_f0 = md.k.freq_start_hz;
+    ctx->tab->lambda_df = md.k.freq_inc_hz;
+    LEAP_CUDA(cudaMemcpyAsync(ctx->tab->lambda.ptr, ctx->tab->lambda_host.data(), sizeof(double) * 2 * channels,
                               cudaMemcpyHostToDevice, s),
               "upload wavelengths");
-    ctx->fx_rho_host.resize(channels);
-    ctx->fx_ok = fx_spectrum(md.k.freq_start_hz, md.k.freq_inc_hz, channels, ctx->lambda_host.data(), ctx->fx_sp,
-                             ctx->fx_rho_host.data());
-    if (ctx->fx_ok) {
-      LEAP_CUDA(ctx->fx_rho.ensure(sizeof(int32_t) * channels), "alloc wavelength corrections");
-      LEAP_CUDA(cudaMemcpyAsync(ctx->fx_rho.ptr, ctx->fx_rho_host.data(), sizeof(int32_t) * channels,
+    ctx->tab->fx_rho_host.resize(channels);
+    ctx->tab->fx_ok = fx_spectrum(md.k.freq_start_hz, md.k.freq_inc_hz, channels, ctx->tab->lambda_host.data(), ctx->tab->fx_sp,
+                             ctx->tab->fx_rho_host.data());
+    if (ctx->tab->fx_ok) {
+      LEAP_CUDA(ctx->tab->fx_rho.ensure(sizeof(int32_t) * channels), "alloc wavelength corrections");
+      LEAP_CUDA(cudaMemcpyAsync(ctx->tab->fx_rho.ptr, ctx->tab->fx_rho_host.data(), sizeof(int32_t) * channels,
                                 cudaMemcpyHostToDevice, s),
                 "upload wavelength corrections");
     }
@@ -417,19 +425,19 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
       }
       std::vector<int32_t>& order = ctx->pipe_order_host;
       schedule_units(std::move(runs), grid, order);
-      LEAP_CUDA(ctx->pipe_order.ensure(sizeof(int32_t) * order.size()), "alloc unit order");
+      LEAP_CUDA(ctx->tab->pipe_order.ensure(sizeof(int32_t) * order.size()), "alloc unit order");
       if (!ctx->capturing)
-        LEAP_CUDA(cudaMemcpyAsync(ctx->pipe_order.ptr, order.data(), sizeof(int32_t) * order.size(),
+        LEAP_CUDA(cudaMemcpyAsync(ctx->tab->pipe_order.ptr, order.data(), sizeof(int32_t) * order.size(),
                                   cudaMemcpyHostToDevice, s),
                   "upload unit order");
     }
-    LEAP_CUDA(ctx->pipe_items.ensure(sizeof(PipeItem) * pit.size()), "alloc item table");
+    LEAP_CUDA(ctx->tab->pipe_items.ensure(sizeof(PipeItem) * pit.size()), "alloc item table");
     if (!ctx->capturing)
-      LEAP_CUDA(cudaMemcpyAsync(ctx->pipe_items.ptr, pit.data(), sizeof(PipeItem) * pit.size(), cudaMemcpyHostToDevice, s),
+      LEAP_CUDA(cudaMemcpyAsync(ctx->tab->pipe_items.ptr, pit.data(), sizeof(PipeItem) * pit.size(), cudaMemcpyHostToDevice, s),
                 "upload item table");
     if (!red.empty() && !ctx->capturing) {
-      LEAP_CUDA(ctx->reduce_items.ensure(sizeof(ReduceItem) * red.size()), "alloc reduce table");
-      LEAP_CUDA(cudaMemcpyAsync(ctx->reduce_items.ptr, red.data(), sizeof(ReduceItem) * red.size(),
+      LEAP_CUDA(ctx->tab->reduce_items.ensure(sizeof(ReduceItem) * red.size()), "alloc reduce table");
+      LEAP_CUDA(cudaMemcpyAsync(ctx->tab->reduce_items.ptr, red.data(), sizeof(ReduceItem) * red.size(),
                                 cudaMemcpyHostToDevice, s),
                 "upload reduce table");
     }
@@ -437,8 +445,8 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
                                                      ctx->dirk.as<float>());
     ++kernels;
     PipeParams pp{};
-    pp.items = ctx->pipe_items.as<PipeItem>();
-    pp.order = ctx->pipe_order.as<int32_t>();
+    pp.items = ctx->tab->pipe_items.as<PipeItem>();
+    pp.order = ctx->tab->pipe_order.as<int32_t>();
     pp.nslots = static_cast<int32_t>(ctx->pipe_order_host.size());
     pp.nitems = static_cast<int32_t>(pit.size());
     pp.units = units;
@@ -464,7 +472,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
       int64_t maxn = 0;
       for (const auto& r : red) maxn = std::max<int64_t>(maxn, static_cast<int64_t>(r.ndir) * 4 * nbl);
       const dim3 rg(static_cast<unsigned>(std::min<int64_t>((maxn + 255) / 256, 1024)), static_cast<unsigned>(red.size()));
-      reduce_item_slabs<<<rg, 256, 0, s>>>(ctx->reduce_items.as<ReduceItem>(), static_cast<int>(red.size()), 4 * nbl,
+      reduce_item_slabs<<<rg, 256, 0, s>>>(ctx->tab->reduce_items.as<ReduceItem>(), static_cast<int>(red.size()), 4 * nbl,
                                             ctx->avg.as<double2>());
       ++kernels;
     }
@@ -476,7 +484,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     Integration& in = ctx->integ.at(w.slot);
     const int T = static_cast<int>(in.rows / nbl);
     const int C = in.channels;
-    const bool fixed = precision == LEAP_PRECISION_FP64 && ctx->fx_ok;
+    const bool fixed = precision == LEAP_PRECISION_FP64 && ctx->tab->fx_ok;
     int dirs_per_block = precision == LEAP_PRECISION_FP64 ? 8 : 16;  // 4 warps of 2 or 4 directions
     int nw = 4;
     if (fixed) {
@@ -503,8 +511,8 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     ra.vis = in.vis.ptr;
     ra.uvw = in.uvw.as<double>();
     ra.dd = d_dd + 9 * static_cast<int64_t>(w.dir0);
-    ra.lambda = ctx->lambda.as<double>();
-    ra.inv_lambda = ctx->lambda.as<double>() + ctx->lambda_host.size() / 2;
+    ra.lambda = ctx->tab->lambda.as<double>();
+    ra.inv_lambda = ctx->tab->lambda.as<double>() + ctx->tab->lambda_host.size() / 2;
     ra.twiddle = ctx->twiddle.as<float2>();
     ra.rows = in.rows;
     ra.channels = C;
@@ -523,7 +531,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     ra.err = ctx->dev_err.as<int>();
     if (fixed) {
       LEAP_CUDA(ctx->fx_exp.ensure(sizeof(int16_t) * in.rows * P), "alloc row exponents");
-      FxArgs fa{ra, ctx->fx_sp, ctx->fx_tab.as<int4>(), ctx->fx_rho.as<int32_t>(), ctx->fx_exp.as<int16_t>()};
+      FxArgs fa{ra, ctx->tab->fx_sp, ctx->fx_tab.as<int4>(), ctx->tab->fx_rho.as<int32_t>(), ctx->fx_exp.as<int16_t>()};
       const int rc = dispatch_fixed(ctx, in.vis_type, fa, nw, dim3(tiles * dgroups, nslab), s);
       if (rc != LEAP_OK) return rc;
       ++kernels;
@@ -550,7 +558,7 @@ int refant_reduce(leap_ctx* ctx, cudaStream_t st, int& kernels) {
   int64_t maxn = 0;
   for (const auto& r : red) maxn = std::max<int64_t>(maxn, static_cast<int64_t>(r.ndir) * nI1);
   const dim3 rg(static_cast<unsigned>(std::min<int64_t>((maxn + 255) / 256, 1024)), static_cast<unsigned>(red.size()));
-  reduce_item_slabs<<<rg, 256, 0, st>>>(ctx->refant_reduce.as<ReduceItem>(), static_cast<int>(red.size()), nI1,
+  reduce_item_slabs<<<rg, 256, 0, st>>>(ctx->tab->refant_reduce.as<ReduceItem>(), static_cast<int>(red.size()), nI1,
                                          ctx->avg_i1.as<double2>());
   ++kernels;
   return LEAP_OK;
@@ -605,8 +613,8 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
       rr.vis = in.vis.ptr;
       rr.uvw = in.uvw.as<double>();
       rr.dd = d_dd + 9 * static_cast<int64_t>(w.dir0);
-      rr.lambda = ctx->lambda.as<double>();
-      rr.inv_lambda = ctx->lambda.as<double>() + ctx->lambda_host.size() / 2;
+      rr.lambda = ctx->tab->lambda.as<double>();
+      rr.inv_lambda = ctx->tab->lambda.as<double>() + ctx->tab->lambda_host.size() / 2;
       rr.rows = in.rows;
       rr.channels = in.channels;
       rr.pols = in.pols;
@@ -662,18 +670,18 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     rit[i].out = ctx->partial_i1.as<double2>() + off[i];
     red[i].partial = rit[i].out;
   }
-  LEAP_CUDA(ctx->refant_items.ensure(sizeof(RefantItem) * rit.size()), "alloc refant table");
-  LEAP_CUDA(ctx->refant_reduce.ensure(sizeof(ReduceItem) * red.size()), "alloc refant reduce table");
+  LEAP_CUDA(ctx->tab->refant_items.ensure(sizeof(RefantItem) * rit.size()), "alloc refant table");
+  LEAP_CUDA(ctx->tab->refant_reduce.ensure(sizeof(ReduceItem) * red.size()), "alloc refant reduce table");
   if (!ctx->capturing) {
-    LEAP_CUDA(cudaMemcpyAsync(ctx->refant_items.ptr, rit.data(), sizeof(RefantItem) * rit.size(), cudaMemcpyHostToDevice,
+    LEAP_CUDA(cudaMemcpyAsync(ctx->tab->refant_items.ptr, rit.data(), sizeof(RefantItem) * rit.size(), cudaMemcpyHostToDevice,
                               a),
               "upload refant table");
-    LEAP_CUDA(cudaMemcpyAsync(ctx->refant_reduce.ptr, red.data(), sizeof(ReduceItem) * red.size(),
+    LEAP_CUDA(cudaMemcpyAsync(ctx->tab->refant_reduce.ptr, red.data(), sizeof(ReduceItem) * red.size(),
                               cudaMemcpyHostToDevice, a),
               "upload refant reduce table");
   }
   RefantParams rp{};
-  rp.items = ctx->refant_items.as<RefantItem>();
+  rp.items = ctx->tab->refant_items.as<RefantItem>();
   rp.I1 = md.I1.as<int32_t>();
   rp.f0 = md.k.freq_start_hz;
   rp.df = md.k.freq_inc_hz;
@@ -944,22 +952,65 @@ int autotune_batch(leap_ctx* ctx, const std::vector<WorkItem>& items, int32_t D,
   return LEAP_OK;
 }
 
+// Everything that a recorded batched call has fixed besides buffer addresses: its launches and tables follow from the
+// key, the metadata, and the shape of each slot.  Empty where a slot is not set (the call is refused).
+std::string graph_signature(const leap_ctx* ctx, const std::vector<WorkItem>& items, const std::string& key) {
+  std::string k = key + "|md" + std::to_string(ctx->md_gen);
+  for (const auto& w : items) {
+    auto it = ctx->integ.find(w.slot);
+    if (it == ctx->integ.end()) return {};
+    const Integration& in = it->second;
+    k += "|" + std::to_string(in.rows) + "," + std::to_string(in.channels) + "," + std::to_string(in.pols) + "," +
+         std::to_string(in.vis_type) + (in.has_map ? "m" : "");
+  }
+  return k;
+}
+
+// Replays the recorded call on what the slots hold now; `done` tells whether it could be.  The split operand of a new
+// integration is not part of the graph.
+int replay_batched(leap_ctx* ctx, const std::vector<WorkItem>& items, int32_t D, int32_t precision, bool& done) {
+  cudaStream_t s = ctx->stream;
+  const int P = ctx->integ.at(items[0].slot).pols;
+  wait_for_uploads(ctx, items, s);
+  cudaEvent_t* ev = ctx->ring[ctx->ring_count % leap_ctx::kRing];
+  cudaEventRecord(ev[0], s);
+  if (uses_gridded(ctx, items, D, precision, P)) {
+    int kernels = 0;
+    for (const auto& w : items)
+      if (const int rc = ensure_grid_operand(ctx, ctx->integ.at(w.slot), s, kernels)) return rc;
+  }
+  done = ctx->graph_epoch == g_alloc_epoch;
+  if (!done) return LEAP_OK;
+  cudaEventRecord(ev[1], s);
+  LEAP_CUDA(cudaGraphLaunch(ctx->graph_exec, s), "graph launch");
+  cudaEventRecord(ev[2], s);
+  ctx->ring_count++;
+  ctx->last_ndir = D;
+  ctx->last_pols = P;
+  ctx->last_nbl = static_cast<int32_t>(ctx->md.k.nbaselines);
+  ctx->kernels_last = ctx->graph_kernels;
+  return LEAP_OK;
+}
+
 int calibrate_batched_impl(leap_ctx* ctx, const leap_work_item* witems, int32_t nitems, int32_t D, int32_t precision) {
   if (!witems || nitems <= 0) return fail(ctx, LEAP_ERR_INVALID_ARGUMENT, "no work items");
   std::vector<WorkItem> items(nitems);
   for (int i = 0; i < nitems; ++i) items[i] = WorkItem{witems[i].slot, witems[i].first_direction, witems[i].ndirections};
   const std::string key = batch_key(ctx, items, D, precision);
   cudaStream_t s = ctx->stream;
-  if (ctx->graph_replay && ctx->graph_exec && ctx->graph_key == key && ctx->graph_epoch == g_alloc_epoch) {
-    wait_for_uploads(ctx, items, s);
-    cudaEvent_t* ev = ctx->ring[ctx->ring_count % leap_ctx::kRing];
-    cudaEventRecord(ev[0], s);
-    cudaEventRecord(ev[1], s);
-    LEAP_CUDA(cudaGraphLaunch(ctx->graph_exec, s), "graph launch");
-    cudaEventRecord(ev[2], s);
-    ctx->ring_count++;
-    return LEAP_OK;
+  const std::string sig = graph_signature(ctx, items, key);
+  if (ctx->graph_replay && !sig.empty() && ctx->graph_sig == sig) {
+    bool done = false;
+    const int rc = replay_batched(ctx, items, D, precision, done);
+    if (rc != LEAP_OK || done) return rc;
   }
+  // From here on the tables that the graph reads are rewritten.
+  ctx->graph_sig.clear();
+  struct OwnTables {
+    leap_ctx* ctx;
+    explicit OwnTables(leap_ctx* c) : ctx(c) { ctx->tab = &ctx->batched; }
+    ~OwnTables() { ctx->tab = &ctx->single; }
+  } own(ctx);
   auto t = ctx->tuned.find(key);
   if (t != ctx->tuned.end()) {
     ctx->tune = t->second;
@@ -991,8 +1042,9 @@ int calibrate_batched_impl(leap_ctx* ctx, const leap_work_item* witems, int32_t 
   const cudaError_t ei = cudaGraphInstantiate(&ctx->graph_exec, graph, 0);
   cudaGraphDestroy(graph);
   if (ei != cudaSuccess) return cuda_fail(ctx, ei, "instantiate graph");
-  ctx->graph_key = key;
+  ctx->graph_sig = sig;
   ctx->graph_epoch = g_alloc_epoch;
+  ctx->graph_kernels = kernels;
   return LEAP_OK;
 }
 

@@ -132,13 +132,13 @@ void leap_destroy(leap_ctx* ctx) {
     md.at_ptr.release(); md.at_idx.release(); md.at_val.release();
     ctx->dphi_tc.release();
     ctx->partial.release(); ctx->avg.release(); ctx->cal1.release(); ctx->dphi.release();
-    ctx->gemm_partial.release(); ctx->dd.release(); ctx->cal.release(); ctx->dev_err.release(); ctx->lambda.release();
+    ctx->gemm_partial.release(); ctx->dd.release(); ctx->cal.release(); ctx->dev_err.release();
     ctx->dirk.release();
     ctx->twiddle.release();
     ctx->twiddle_df.release();
-    ctx->fx_tab.release(); ctx->fx_rho.release(); ctx->fx_exp.release();
+    ctx->fx_tab.release(); ctx->fx_exp.release();
     for (auto& kv : ctx->grid_tabs) kv.second.release();
-    ctx->grid_items.release(); ctx->grid_order.release(); ctx->grid_win.release();
+    ctx->grid_win.release();
     for (auto& tri : ctx->ring)
       for (auto& ev : tri)
         if (ev) cudaEventDestroy(ev);
@@ -156,11 +156,8 @@ void leap_destroy(leap_ctx* ctx) {
     if (ctx->join) cudaEventDestroy(ctx->join);
     ctx->partial_i1.release();
     ctx->avg_i1.release();
-    ctx->pipe_items.release();
-    ctx->pipe_order.release();
-    ctx->reduce_items.release();
-    ctx->refant_items.release();
-    ctx->refant_reduce.release();
+    ctx->single.release();
+    ctx->batched.release();
     ctx->adj_dphi.release(); ctx->adj_cal1.release(); ctx->adj_phi1.release(); ctx->adj_gavg.release();
     ctx->adj_partial.release(); ctx->adj_g.release(); ctx->adj_gexp.release();
     ctx->flag_count.release();

@@ -113,6 +113,22 @@ struct TuneChoice {
   int mma = -1;   // 1: tensor-core (mma.sync) bulk kernel, 0: CUDA-core kernel, -1: by direction count
 };
 
+// What a call's kernels read besides its inputs: launch tables, and per-channel constants of the spectral window.
+struct LaunchTables {
+  DeviceBuffer pipe_items, pipe_order, grid_items, grid_order, reduce_items, refant_items, refant_reduce;
+  DeviceBuffer lambda, fx_rho;        // wavelengths and their reciprocals; corrections of the fixed-point phasors
+  std::vector<double> lambda_host;
+  double lambda_f0 = 0.0, lambda_df = 0.0;
+  std::vector<int32_t> fx_rho_host;
+  FxSpectrum fx_sp{};
+  bool fx_ok = false;                 // the fixed-point phasors apply to this window
+  void release() {
+    for (DeviceBuffer* b : {&pipe_items, &pipe_order, &grid_items, &grid_order, &reduce_items, &refant_items,
+                            &refant_reduce, &lambda, &fx_rho})
+      b->release();
+  }
+};
+
 struct leap_ctx {
   int device = 0;
   int sms = 152;
@@ -132,7 +148,7 @@ struct leap_ctx {
   std::map<int, float> grid_einv;         // ... and the inverse of its scale
   std::vector<GridItem> grid_items_host;
   std::vector<int32_t> grid_order_host;
-  DeviceBuffer grid_items, grid_order, grid_win;
+  DeviceBuffer grid_win;
   bool pipe_attr_mma = false;
   bool refant_attr_set = false;       // its shared-memory size was raised
   int tc_attr_set = 0;                // bit per N tile whose shared-memory size was raised
@@ -146,34 +162,32 @@ struct leap_ctx {
   DeviceBuffer stage_dev[2];
   cudaEvent_t stage_done[2] = {nullptr, nullptr};
   std::map<std::string, TuneChoice> tuned;
-  std::string graph_key;
+  // The recorded batched call: replayed for calls of the same signature (graph_signature) while no buffer moves.
+  std::string graph_sig;              // empty: nothing to replay
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_epoch = 0;
+  int graph_kernels = 0;
+  uint64_t md_gen = 0;                // counts the metadata installed
   std::vector<PipeItem> pipe_items_host;
   std::vector<int32_t> pipe_order_host;
   std::vector<ReduceItem> reduce_items_host, refant_reduce_host;
   std::vector<RefantItem> refant_items_host;
-  DeviceBuffer pipe_items, pipe_order, reduce_items, refant_items, refant_reduce;
+  // Batched calls have tables of their own, which their recorded graph goes on reading: other calls do not write them.
+  LaunchTables single, batched;
+  LaunchTables* tab = &single;        // those of the call being made
   cudaStream_t stream = nullptr;
   std::string err;
   Metadata md;
   std::map<int32_t, Integration> integ;
   // scratch, shared by calls on this context
-  DeviceBuffer partial, avg, cal1, dphi, gemm_partial, dd, cal, dev_err, lambda, twiddle, twiddle_df, partial_i1, avg_i1,
-      dirk;
+  DeviceBuffer partial, avg, cal1, dphi, gemm_partial, dd, cal, dev_err, twiddle, twiddle_df, partial_i1, avg_i1, dirk;
   cudaStream_t aux = nullptr;           // second stream for the FP64 reference-antenna pass
   cudaStream_t copy = nullptr;          // asynchronous ingestion
   cudaEvent_t copy_fence = nullptr;     // orders an asynchronous upload after earlier calls
   cudaEvent_t fork = nullptr, join = nullptr;
   int last_ndir = 0, last_pols = 0, last_nbl = 0;
-  std::vector<double> lambda_host;
-  double lambda_f0 = 0.0, lambda_df = 0.0;
-  // Fixed-point phasors of the all-FP64 form: tables, per-channel corrections, the spectral window
-  // (fx_ok: it applies), and the row exponents of the item being rotated.
-  DeviceBuffer fx_tab, fx_rho, fx_exp;
-  std::vector<int32_t> fx_rho_host;
-  FxSpectrum fx_sp{};
-  bool fx_ok = false;
+  // Fixed-point phasors of the all-FP64 form: tables, and the row exponents of the item being rotated.
+  DeviceBuffer fx_tab, fx_exp;
   uint32_t fx_attr_set = 0;           // bit per kernel variant whose shared-memory size was raised
   // Ring of (start, after rotate, end) events, one triple per recorded call.
   static constexpr int kRing = 256;

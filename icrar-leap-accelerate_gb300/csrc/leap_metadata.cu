@@ -18,6 +18,7 @@ int install_metadata(leap_ctx* ctx, const leap_constants* k, const std::vector<i
   }
   Metadata& md = ctx->md;
   md.set = false;
+  ++ctx->md_gen;
   md.k = *k;
   md.S = A_cols;
   md.Arows = A_rows;
