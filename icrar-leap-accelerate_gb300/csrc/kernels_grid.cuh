@@ -345,6 +345,13 @@ __device__ __forceinline__ bool grid_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// The same by a whole warp, with one outcome for all of its lanes: each lane polls on its own, and the abort flag or the
+// limit may reach some of them before the barrier's phase does, but the role's shuffles, warp barriers and warp-wide
+// tcgen05 instructions need every lane to go on, or every lane to leave.
+__device__ __forceinline__ bool grid_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, grid_wait(bar, parity, abort_flag));
+}
+
 __device__ __forceinline__ void grid_fail(const GridParams& p, volatile int* abort_flag) {
   atomicOr(p.err, kDevErrTimeout);
   *abort_flag = 1;
@@ -871,8 +878,8 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
       for (int tb = 0; tb < ntb && ok; ++tb)
         for (int ps = 0; ps < npass && ok; ++ps, ++blk) {
           const uint32_t b = blk & 1;
-          if ((blk >= 2 && !grid_wait(&rs_free[b], ((blk >> 1) - 1) & 1, abort_flag)) ||
-              (blk >= 1 && !grid_wait(ac_free, (blk - 1) & 1, abort_flag))) {
+          if ((blk >= 2 && !grid_wait_warp(&rs_free[b], ((blk >> 1) - 1) & 1, abort_flag)) ||
+              (blk >= 1 && !grid_wait_warp(ac_free, (blk - 1) & 1, abort_flag))) {
             if (lead) grid_fail(p, abort_flag);
             ok = false;
             break;
@@ -882,7 +889,7 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
           for (int q0 = 0; q0 < nchunk && ok; q0 += kGrMacro, ++ctr) {
             const int m = ctr % kGrMacroStages;
             const int nq = min(kGrMacro, nchunk - q0);
-            if (!grid_wait(&vfull[m], (ctr / kGrMacroStages) & 1, abort_flag)) {
+            if (!grid_wait_warp(&vfull[m], (ctr / kGrMacroStages) & 1, abort_flag)) {
               if (lead) grid_fail(p, abort_flag);
               ok = false;
               break;
@@ -904,7 +911,7 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
                                        ed + i * est + (256 >> 4), idesc, q0 + i > 0 ? 1u : 0u);
             }
             issued = true;
-            if (seg >= 2 && !grid_wait(is_empty, (mids - 1) & 1, abort_flag)) {
+            if (seg >= 2 && !grid_wait_warp(is_empty, (mids - 1) & 1, abort_flag)) {
               if (lead) grid_fail(p, abort_flag);
               ok = false;
             } else {
@@ -947,7 +954,7 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
           // segment can restart IS.  (Segment 0 accumulates in RS itself.)
           for (int sg = 1; sg <= nseg - 2; ++sg) {
             const uint32_t r = rnd + sg;
-            if (!grid_wait(&sdone[r % kGrMacroStages], (r / kGrMacroStages) & 1, abort_flag)) {
+            if (!grid_wait_warp(&sdone[r % kGrMacroStages], (r / kGrMacroStages) & 1, abort_flag)) {
               grid_fail(p, abort_flag);
               ok = false;
               break;
@@ -961,8 +968,8 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
           if (!ok) break;
           // Final fold: RS += last segment (if any beyond the first) + corrections.
           const uint32_t rl = rnd + nseg - 1;  // the tile's last round: every MMA of the tile completed
-          if ((blk >= 2 && !grid_wait(&rs_free[b], ((blk >> 1) - 1) & 1, abort_flag)) ||
-              !grid_wait(&sdone[rl % kGrMacroStages], (rl / kGrMacroStages) & 1, abort_flag)) {
+          if ((blk >= 2 && !grid_wait_warp(&rs_free[b], ((blk >> 1) - 1) & 1, abort_flag)) ||
+              !grid_wait_warp(&sdone[rl % kGrMacroStages], (rl / kGrMacroStages) & 1, abort_flag)) {
             grid_fail(p, abort_flag);
             ok = false;
             break;
@@ -1023,7 +1030,7 @@ __global__ void __launch_bounds__(kGrThreads, 1) rotate_average_gridded(const Gr
         for (int i = 0; i < 6; ++i) x[i] = __ldg(I.uvw_f + 6 * r + i);
         for (int pp = 0; pp < w.npass; ++pp, ++blk) {
           const uint32_t rb = blk & 1;
-          if (!grid_wait(&rs_full[rb], (blk >> 1) & 1, abort_flag)) {
+          if (!grid_wait_warp(&rs_full[rb], (blk >> 1) & 1, abort_flag)) {
             grid_fail(p, abort_flag);
             ok = false;
             break;
