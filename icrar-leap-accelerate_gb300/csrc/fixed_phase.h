@@ -269,4 +269,42 @@ LEAP_HD void fx_step(int64_t& re, int64_t& im, const FxLimbs& w, int32_t d, int3
              turned, re, im);
 }
 
+// A component in [-1, 1] (to a scale) as (h + l 2^-32) 2^-28: h at most 2^28, l a signed 32-bit remainder.
+struct FxPart {
+  int32_t h, l;
+};
+
+// Of a 60-bit fixed-point number.
+LEAP_HD FxPart fx_part(int64_t z) {
+  const int32_t l = static_cast<int32_t>(static_cast<uint32_t>(z));
+  return FxPart{static_cast<int32_t>((z + (int64_t(1) << 31)) >> 32), l};
+}
+
+// Of x, at most 2^28 in absolute value, to 2^-32.  (-l is one too.)
+LEAP_HD FxPart fx_part(double x) {
+  FxPart r;
+#ifdef __CUDA_ARCH__
+  r.h = __double2int_rn(x);
+  r.l = __double2int_rn((x - r.h) * 4294967296.0);  // 2^31 saturates
+#else
+  r.h = static_cast<int32_t>(__builtin_nearbyint(x));
+  const double l = __builtin_nearbyint((x - r.h) * 4294967296.0);
+  r.l = l > 2147483647.0 ? 2147483647 : static_cast<int32_t>(l);
+#endif
+  if (r.l < -2147483647) r.l = -2147483647;
+  return r;
+}
+
+// sum += a x + b y in units of 2^-56: the products of the high parts exactly, those of a high and a low part rounded
+// together to the unit, those of the low parts (below half a unit) dropped.
+LEAP_HD void fx_add_products(int64_t& sum, const FxPart& a, const FxPart& x, const FxPart& b, const FxPart& y) {
+  int64_t mid = fx_mul(a.h, x.l);
+  fx_mad(sum, a.h, x.h);
+  fx_mad(mid, a.l, x.h);
+  fx_mad(sum, b.h, y.h);
+  fx_mad(mid, b.h, y.l);
+  fx_mad(mid, b.l, y.h);
+  sum += static_cast<int32_t>((mid + (int64_t(1) << 31)) >> 32);
+}
+
 }  // namespace leapgb

@@ -206,7 +206,7 @@ struct AdjointFixedArgs {
   const int16_t* vexp;       // [rows] (adjoint_exponents)
   int32_t kexp;              // 1 / lambda < 2^kexp
   int32_t T, t_per_slab, n_tslab, c_per_slab, n_cslab;
-  const int4* g;             // [D][nbl] split g_avg (adjoint_split_g)
+  const int4* g;             // [D][nbl][2] split g_avg (adjoint_split_g)
   const int16_t* gexp;       // [nbl]
 };
 
@@ -356,9 +356,8 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) adjoint_lmn_fixed(const Adjo
     }
 }
 
-// g_avg in limbs, for adjoint_vis_fixed: g 2^(28 - e) = h + l for both components, |l| <= 1/2, with e such that
-// the sums of D products stay below 2^63 (65 directions and more give up a bit per doubling).  e = kFxPlain: a
-// gradient that is not finite, or out of range.
+// g_avg for adjoint_vis_fixed: two words of four per (direction, baseline), g 2^(28 - e) in parts (re, im), then -re.
+// e = kFxPlain: a gradient that is not finite, or out of range.
 static __global__ void adjoint_split_g(const double2* __restrict__ gavg, int nbl, int D, int4* __restrict__ out,
                                        int16_t* __restrict__ gexp) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -368,17 +367,16 @@ static __global__ void adjoint_split_g(const double2* __restrict__ gavg, int nbl
     const double2 g = gavg[static_cast<int64_t>(d) * nbl + b];
     m = max(m, max(fx_magnitude(g.x), fx_magnitude(g.y)));
   }
-  int e = fx_exponent<double2>(m);
+  const int e = fx_exponent<double2>(m);
   const bool plain = e == kFxPlain;
-  for (int q = 64; q < D; q *= 2) ++e;
-  gexp[b] = static_cast<int16_t>(plain ? kFxPlain : e);
+  gexp[b] = static_cast<int16_t>(e);
   const double scale = plain ? 0.0 : scalbn(1.0, 28 - e);
   for (int d = 0; d < D; ++d) {
-    const double2 g = gavg[static_cast<int64_t>(d) * nbl + b];
-    const double x = g.x * scale, y = g.y * scale;
-    const int hx = plain ? 0 : __double2int_rn(x), hy = plain ? 0 : __double2int_rn(y);
-    const float lx = plain ? 0.f : static_cast<float>(x - hx), ly = plain ? 0.f : static_cast<float>(y - hy);
-    out[static_cast<int64_t>(d) * nbl + b] = make_int4(hx, __float_as_int(lx), hy, __float_as_int(ly));
+    const int64_t i = static_cast<int64_t>(d) * nbl + b;
+    const double2 g = gavg[i];
+    const FxPart x = fx_part(plain ? 0.0 : g.x * scale), y = fx_part(plain ? 0.0 : g.y * scale);
+    out[2 * i] = make_int4(x.h, x.l, y.h, y.l);
+    out[2 * i + 1] = make_int4(-x.h, -x.l, 0, 0);
   }
 }
 
@@ -402,17 +400,23 @@ __device__ __forceinline__ void adj_write(float2* dst, double re, double im) { *
 __device__ __forceinline__ void adj_write(double2* dst, double re, double im) { *dst = make_double2(re, im); }
 
 // g_V[0][r][c] = sum_d g_avg[d][b] exp(-i phase_d[r][c]) and zeros for the other pols, zero at dropped groups.  A
-// warp takes 32 rows (lanes) and kVisChannels channels, whose sums it keeps over the directions: h h in 64 bits, h l
-// and l h in FP32, as FxSumFloat.  128 antennas, 8 timesteps, 96 channels, 16 directions: 3.04 -> 0.69 ms (FP64
-// FMAs: 8 per (row, channel, direction) and two sincos per 16 channels).
+// warp takes 32 rows (lanes) and kVisChannels channels, whose sums over the directions it keeps in 64-bit integers
+// (fx_add_products), added to FP64 sums in shared memory every kVisFlush directions where there are more.  128
+// antennas, 8 timesteps, 96 channels, 16 directions: 3.04 -> 0.64 ms (FP64 FMAs: 8 per (row, channel, direction) and
+// two sincos per 16 channels).
 constexpr int kVisChannels = 16;
+constexpr int kVisFlush = 64;  // sqrt(2) 2^56 units a direction at most: below 2^63
+constexpr int kVisThreads = 128;
+constexpr int kVisSumBytes = kVisChannels * kVisThreads * 16;
 template <typename VisT, int P>
-__global__ void __launch_bounds__(128, 3) adjoint_vis_fixed(const AdjointFixedArgs f) {
+__global__ void __launch_bounds__(kVisThreads, 3) adjoint_vis_fixed(const AdjointFixedArgs f) {
+  extern __shared__ __align__(128) unsigned char fx_smem[];
+  double2* sums = reinterpret_cast<double2*>(fx_smem) + threadIdx.x;  // [kVisChannels][kVisThreads]: with more than kVisFlush directions
   const AdjointArgs& a = f.a;
   const int lane = threadIdx.x & 31;
   const int ncb = (a.C + kVisChannels - 1) / kVisChannels;
   const int64_t rtiles = (a.rows + 31) / 32;
-  const int64_t unit = blockIdx.x * 4ll + (threadIdx.x >> 5);
+  const int64_t unit = blockIdx.x * static_cast<int64_t>(kVisThreads / 32) + (threadIdx.x >> 5);
   if (unit >= rtiles * ncb) return;
   const int c0 = static_cast<int>(unit % ncb) * kVisChannels, n = min(kVisChannels, a.C - c0);
   const int64_t r = (unit / ncb) * 32 + lane;
@@ -422,31 +426,33 @@ __global__ void __launch_bounds__(128, 3) adjoint_vis_fixed(const AdjointFixedAr
   const int ge = __ldg(f.gexp + b);
   bool plain = ge == kFxPlain;
   int64_t hr[kVisChannels], hi[kVisChannels];
-  float mr[kVisChannels], mi[kVisChannels];
 #pragma unroll
-  for (int k = 0; k < kVisChannels; ++k) {
-    hr[k] = hi[k] = 0;
-    mr[k] = mi[k] = 0.f;
-  }
+  for (int k = 0; k < kVisChannels; ++k) hr[k] = hi[k] = 0;
   const double u = __ldg(a.uvw + 3 * rr), v = __ldg(a.uvw + 3 * rr + 1), w = __ldg(a.uvw + 3 * rr + 2);
   for (int d = 0; d < a.D; ++d) {
-    const int4 g = __ldg(f.g + static_cast<int64_t>(d) * a.nbl + b);
+    if (d > 0 && d % kVisFlush == 0) {
+#pragma unroll
+      for (int k = 0; k < kVisChannels; ++k) {
+        double2 s = make_double2(static_cast<double>(hr[k]), static_cast<double>(hi[k]));
+        if (d > kVisFlush) {
+          s.x += sums[k * kVisThreads].x;
+          s.y += sums[k * kVisThreads].y;
+        }
+        sums[k * kVisThreads] = s;
+        hr[k] = hi[k] = 0;
+      }
+    }
+    const int4* g = f.g + 2 * (static_cast<int64_t>(d) * a.nbl + b);
+    const int4 g0 = __ldg(g), g1 = __ldg(g + 1);
+    const FxPart gx{g0.x, g0.y}, gy{g0.z, g0.w}, ngx{g1.x, g1.y};
     FxRay ray;
     plain |= !ray.begin(fx_shift_factor(a.dd + 9 * d + 6, u, v, w), f.sp, c0, f.tab);
     ray.seed(__ldg(f.rho + c0), f.tab);
-    constexpr float kUnit = FxSumFloat<1>::kUnit;
-    const float lx = __int_as_float(g.y), ly = __int_as_float(g.w), hx = g.x * kUnit, hy = g.z * kUnit;
 #pragma unroll
     for (int k = 0; k < kVisChannels; ++k) {
-      const typename FxSumFloat<1>::Phasor z = FxSumFloat<1>::phasor(ray.zr, ray.zi);
-      fx_mad(hr[k], g.x, z.rh);  // re: g.x z.r + g.y z.i; im: g.y z.r - g.x z.i
-      fx_mad(hi[k], g.z, z.rh);
-      fx_mad(hr[k], g.z, z.ih);
-      fx_mad(hi[k], g.x, z.nih);
-      mr[k] = fmaf(lx, z.rhf, fmaf(hx, z.rlf, mr[k]));
-      mi[k] = fmaf(ly, z.rhf, fmaf(hy, z.rlf, mi[k]));
-      mr[k] = fmaf(ly, z.ihf, fmaf(hy, z.ilf, mr[k]));
-      mi[k] = fmaf(-lx, z.ihf, fmaf(-hx, z.ilf, mi[k]));
+      const FxPart zr = fx_part(ray.zr), zi = fx_part(ray.zi);
+      fx_add_products(hr[k], gx, zr, gy, zi);   // re: g.x z.r + g.y z.i
+      fx_add_products(hi[k], gy, zr, ngx, zi);  // im: g.y z.r - g.x z.i
       if (k + 1 < kVisChannels) ray.next(__ldg(f.rho + min(c0 + k + 1, a.C - 1)));
     }
   }
@@ -465,7 +471,12 @@ __global__ void __launch_bounds__(128, 3) adjoint_vis_fixed(const AdjointFixedAr
         drop |= isnan(x.x) || isnan(x.y);
       }
     }
-    double2 o = make_double2((static_cast<double>(hr[k]) + mr[k]) * scale, (static_cast<double>(hi[k]) + mi[k]) * scale);
+    double2 o = make_double2(static_cast<double>(hr[k]), static_cast<double>(hi[k]));
+    if (a.D > kVisFlush) {
+      o.x += sums[k * kVisThreads].x;
+      o.y += sums[k * kVisThreads].y;
+    }
+    o = make_double2(o.x * scale, o.y * scale);
     if (plain) o = adj_plain_vis(f, r, b, c0 + k);
     if (drop) o = make_double2(0.0, 0.0);
     VisT* dst = static_cast<VisT*>(a.gvis) + base;

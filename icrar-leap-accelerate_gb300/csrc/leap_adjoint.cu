@@ -38,7 +38,9 @@ int adjoint_fixed(leap_ctx* ctx, AdjointFixedArgs fa, double* d_grad_lmn, cudaSt
   if (a.gvis) {
     adjoint_split_g<<<(nbl + 127) / 128, 128, 0, s>>>(a.gavg, nbl, D, const_cast<int4*>(fa.g), const_cast<int16_t*>(fa.gexp));
     const int64_t units = ((a.rows + 31) / 32) * ((a.C + kVisChannels - 1) / kVisChannels);
-    adjoint_vis_fixed<VisT, P><<<static_cast<unsigned>((units + 3) / 4), 128, 0, s>>>(fa);
+    constexpr int warps = kVisThreads / 32;
+    adjoint_vis_fixed<VisT, P><<<static_cast<unsigned>((units + warps - 1) / warps), kVisThreads,
+                                 D > kVisFlush ? kVisSumBytes : 0, s>>>(fa);
   }
   return LEAP_OK;
 }
@@ -110,7 +112,7 @@ int32_t leap_backward(leap_ctx* ctx, int32_t slot, const double* d_dd, int32_t n
   const uintptr_t align = esz * aa.P % 16 == 0 ? 16 : 8;
   if (ctx->tab->fx_ok && in.rows % nbl == 0 && (reinterpret_cast<uintptr_t>(aa.vis) | reinterpret_cast<uintptr_t>(d_grad_vis)) % align == 0) {
     LEAP_CUDA(ctx->fx_exp.ensure(sizeof(int16_t) * in.rows), "alloc row exponents");
-    LEAP_CUDA(ctx->adj_g.ensure(sizeof(int4) * static_cast<size_t>(nbl) * D), "alloc adjoint scratch");
+    LEAP_CUDA(ctx->adj_g.ensure(sizeof(int4) * 2 * static_cast<size_t>(nbl) * D), "alloc adjoint scratch");
     LEAP_CUDA(ctx->adj_gexp.ensure(sizeof(int16_t) * nbl), "alloc adjoint scratch");
     AdjointFixedArgs fa{};
     fa.a = aa;
