@@ -557,4 +557,39 @@ void schedule_units(std::vector<UnitRun> runs, int32_t grid, std::vector<int32_t
   order.resize(order.size() + grid, -1);
 }
 
+// Timesteps may be cut as finely as the call has them, whatever their number: a limit of 32 slabs left 10 antennas, 1000
+// timesteps and one direction with 64 blocks of one warp.  More slabs than 32 of a longer call go on to two rounds of
+// resident blocks only, since their partial sums are added up one after another.
+void choose_fixed_slabs(int timesteps, int channels, int64_t base_blocks, int64_t resident, int& t_per, int& c_per, int& nts,
+                        int& ncs) {
+  double best_eff = 0.0;
+  t_per = timesteps; c_per = channels; nts = ncs = 1;
+  for (int unit : {128, 32, 16}) {
+    const int max_c = (channels + unit - 1) / unit;
+    for (int c = 1; c <= max_c; ++c) {
+      const int cp = ((channels + c - 1) / c + unit - 1) / unit * unit;
+      const int cn = (channels + cp - 1) / cp;
+      if (cn != c) continue;
+      // Slabs of fewer and fewer timesteps; channels are cut only beside slabs of one timestep.
+      for (int t = c == 1 ? 1 : timesteps; t <= timesteps;) {
+        const int tp = (timesteps + t - 1) / t;
+        const int tn = (timesteps + tp - 1) / tp;
+        // Time of the call in blocks' lengths: rounds of resident blocks times a block's samples.
+        const int64_t blocks = base_blocks * cn * tn;
+        if (timesteps > 32 && static_cast<int64_t>(cn) * tn > 32 && blocks > 2 * resident) break;
+        const double rounds = static_cast<double>((blocks + resident - 1) / resident);
+        const double eff = static_cast<double>(base_blocks) * timesteps * channels /
+                           (static_cast<double>(resident) * rounds * tp * std::min(cp, channels));
+        if (eff > best_eff + std::min(0.02, 0.25 * best_eff)) {  // (the share of a small call is small however it is cut)
+          best_eff = eff;
+          t_per = tp; nts = tn; c_per = cp; ncs = cn;
+        }
+        if (best_eff >= 0.95) return;
+        t = tp > 1 ? (timesteps + tp - 2) / (tp - 1) : timesteps + 1;  // the next smaller tp
+      }
+    }
+    if (best_eff >= 0.5) return;
+  }
+}
+
 }  // namespace leapgb

@@ -70,4 +70,12 @@ struct UnitRun {
 // order[k * grid + b] is the k-th unit of block b, or -1 after its last; the last round is all -1.
 void schedule_units(std::vector<UnitRun> runs, int32_t grid, std::vector<int32_t>& order);
 
+// Slab split of (timestep, channel) space for the fixed-point kernels, `resident` of whose blocks run at a time: the
+// fewest slabs whose blocks fill the last round of resident ones to 95%, of whole timesteps, then of 128-channel sums,
+// and of 32-channel blocks (the seeding interval) or 16-channel ones (a stage) only where the call is too small to fill
+// the GPU once (36 antennas, 48 channels, one direction: 145 us a call in 32s, 104 in 16s; in 8s 97, but another small
+// call 8% slower).  t_per and c_per: timesteps and channels of a slab, nts and ncs: slabs.
+void choose_fixed_slabs(int timesteps, int channels, int64_t base_blocks, int64_t resident, int& t_per, int& c_per, int& nts,
+                        int& ncs);
+
 }  // namespace leapgb

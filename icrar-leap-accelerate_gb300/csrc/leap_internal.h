@@ -263,40 +263,6 @@ inline void choose_slabs(int timesteps, int channels, int64_t base_blocks, int& 
   choose_slabs_target(timesteps, channels, base_blocks, 152 * 8, t_per, c_per, nts, ncs);
 }
 
-// Slab split for the fixed-point kernel, `resident` of whose blocks run at a time: the fewest slabs whose
-// blocks fill the last round of resident ones to 95%, of whole timesteps, then of 128-channel sums, and of
-// 32-channel blocks (the seeding interval) or 16-channel ones (a stage) only where the call is too small to fill the
-// GPU once (36 antennas, 48 channels, one direction: 145 us a call in 32s, 104 in 16s; in 8s 97, but another small call
-// 8% slower).
-inline void choose_fixed_slabs(int timesteps, int channels, int64_t base_blocks, int64_t resident, int& t_per, int& c_per,
-                               int& nts, int& ncs) {
-  double best_eff = -1.0;
-  t_per = timesteps; c_per = channels; nts = ncs = 1;
-  for (int unit : {128, 32, 16}) {
-    const int max_c = (channels + unit - 1) / unit;
-    for (int c = 1; c <= max_c; ++c) {
-      const int cp = ((channels + c - 1) / c + unit - 1) / unit * unit;
-      const int cn = (channels + cp - 1) / cp;
-      if (cn != c) continue;
-      for (int t = c == 1 ? 1 : timesteps; t <= std::min(timesteps, 32); ++t) {
-        const int tp = (timesteps + t - 1) / t;
-        const int tn = (timesteps + tp - 1) / tp;
-        // Time of the call in blocks' lengths: rounds of resident blocks times a block's samples.
-        const int64_t blocks = base_blocks * cn * tn;
-        const double rounds = static_cast<double>((blocks + resident - 1) / resident);
-        const double eff = static_cast<double>(base_blocks) * timesteps * channels /
-                           (static_cast<double>(resident) * rounds * tp * std::min(cp, channels));
-        if (eff > best_eff + 0.02) {
-          best_eff = eff;
-          t_per = tp; nts = tn; c_per = cp; ncs = cn;
-        }
-        if (best_eff >= 0.95) return;
-      }
-    }
-    if (best_eff >= 0.5) return;
-  }
-}
-
 // Timestep slabs for the persistent pipelined kernel: the smallest split whose
 // unit count fills the persistent grid to >= 95% on the last round.
 inline void choose_pipe_slabs(int timesteps, int64_t base_units, int grid, int& t_per, int& nts) {
