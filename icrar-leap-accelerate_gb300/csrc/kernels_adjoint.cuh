@@ -234,6 +234,9 @@ __device__ __noinline__ double2 adj_plain_row(const AdjointFixedArgs& f, int64_t
   return s;
 }
 
+template <typename VisT, int P>
+__host__ __device__ constexpr int adjoint_lmn_smem_bytes() { return fx_raw_bytes<VisT, P>() + kFxStage * 32 * 16; }
+
 // dL/d(l, m, n) partial sums.  The forward kernel's structure (kernels_fixed.cuh) for pol 0 times 1 / lambda, with
 // the sums of a row (timestep, baseline) taken to -2 pi Re(conj(g) i S) (u, v, w) at the row's end.  Bound by issue
 // slots as that one is, the recurrence of the phasors above all.  128 antennas, 8 timesteps, 96 channels, 16

@@ -5,25 +5,51 @@
 
 namespace leapabi {
 
-// Rotate + average adjoint in fixed point: dL/d(l, m, n) to d_grad_lmn and, with aa.gvis, dL/dV.
+// Blocks of a variant of the dL/d(l, m, n) kernel that an SM runs at a time: 16 warps by registers (more are not counted),
+// fewer blocks of 1 or 2 warps by shared memory.
 template <typename VisT, int P, int NW>
-int launch_adjoint_lmn(leap_ctx* ctx, const AdjointFixedArgs& fa, dim3 grid, cudaStream_t s) {
-  constexpr int smem = fx_raw_bytes<VisT, P>() + kFxStage * 32 * 16;
-  LEAP_CUDA(cudaFuncSetAttribute(adjoint_lmn_fixed<VisT, P, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-            "set shared memory size");
-  adjoint_lmn_fixed<VisT, P, NW><<<grid, NW * 32, smem, s>>>(fa);
+int adjoint_blocks_nw(leap_ctx* ctx, int& blocks) {
+  constexpr int smem = adjoint_lmn_smem_bytes<VisT, P>();
+  int& n = ctx->adj_blocks[sizeof(VisT) == 8 ? 0 : 1][P / 2][NW == 8 ? 3 : NW / 2];
+  if (n == 0) {
+    LEAP_CUDA(cudaFuncSetAttribute(adjoint_lmn_fixed<VisT, P, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+              "set shared memory size");
+    LEAP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_lmn_fixed<VisT, P, NW>, NW * 32, smem),
+              "query resident blocks");
+    n = std::max(1, std::min(n, 16 / NW));
+  }
+  blocks = n;
   return LEAP_OK;
 }
 
+template <typename VisT, int P, int NW>
+void launch_adjoint_lmn(const AdjointFixedArgs& fa, dim3 grid, cudaStream_t s) {
+  adjoint_lmn_fixed<VisT, P, NW><<<grid, NW * 32, adjoint_lmn_smem_bytes<VisT, P>(), s>>>(fa);
+}
+
+// Rotate + average adjoint in fixed point: dL/d(l, m, n) to d_grad_lmn and, with aa.gvis, dL/dV.
 template <typename VisT, int P>
 int adjoint_fixed(leap_ctx* ctx, AdjointFixedArgs fa, double* d_grad_lmn, cudaStream_t s) {
   const AdjointArgs& a = fa.a;
   const int nbl = a.nbl, D = a.D;
   // Up to 16 directions a block (the split of a stage into limbs is done once for them); fewer, and channel or
   // timestep slabs, as the forward kernel has them.
-  const int nw = D <= 2 ? 1 : D <= 4 ? 2 : D <= 8 ? 4 : 8;
+  int nw = D <= 2 ? 1 : D <= 4 ? 2 : D <= 8 ? 4 : 8;
+  int resident = 1;
+  if (nw == 1) {
+    // 5 blocks of 1 warp (4 complex<double> pols) leave most of the issue slots free (128 antennas, 8 timesteps, 96
+    // channels, 1 direction: 487 us, with 2 warps 434; complex<float>, 9 blocks: 260 and 291).
+    if (const int rc = adjoint_blocks_nw<VisT, P, 1>(ctx, resident)) return rc;
+    if (resident < 8) nw = 2;
+  }
+  {
+    const int rc = nw == 1 ? adjoint_blocks_nw<VisT, P, 1>(ctx, resident) : nw == 2 ? adjoint_blocks_nw<VisT, P, 2>(ctx, resident)
+                 : nw == 4 ? adjoint_blocks_nw<VisT, P, 4>(ctx, resident) : adjoint_blocks_nw<VisT, P, 8>(ctx, resident);
+    if (rc != LEAP_OK) return rc;
+  }
   const int tiles = (nbl + 31) / 32, dgroups = (D + nw * kFxDirs - 1) / (nw * kFxDirs);
-  choose_fixed_slabs(fa.T, a.C, static_cast<int64_t>(tiles) * dgroups, ctx->sms * (16 / nw), fa.t_per_slab, fa.c_per_slab,
+  choose_fixed_slabs(fa.T, a.C, static_cast<int64_t>(tiles) * dgroups, static_cast<int64_t>(ctx->sms) * resident,
+                     fa.t_per_slab, fa.c_per_slab,
                      fa.n_tslab, fa.n_cslab);
   const int nslab = fa.n_tslab * fa.n_cslab, nblk = tiles * nslab;
   LEAP_CUDA(ctx->adj_partial.ensure(sizeof(double) * 3 * static_cast<size_t>(nblk) * D), "alloc adjoint partials");
@@ -31,9 +57,12 @@ int adjoint_fixed(leap_ctx* ctx, AdjointFixedArgs fa, double* d_grad_lmn, cudaSt
   adjoint_exponents<VisT, P><<<static_cast<unsigned>((a.rows + 31) / 32), 256, 0, s>>>(
       static_cast<const VisT*>(a.vis), a.rows, a.C, a.check_nan, const_cast<int16_t*>(fa.vexp));
   const dim3 grid(tiles * dgroups, nslab);
-  const int rc = nw == 1 ? launch_adjoint_lmn<VisT, P, 1>(ctx, fa, grid, s) : nw == 2 ? launch_adjoint_lmn<VisT, P, 2>(ctx, fa, grid, s)
-               : nw == 4 ? launch_adjoint_lmn<VisT, P, 4>(ctx, fa, grid, s) : launch_adjoint_lmn<VisT, P, 8>(ctx, fa, grid, s);
-  if (rc != LEAP_OK) return rc;
+  switch (nw) {
+    case 1: launch_adjoint_lmn<VisT, P, 1>(fa, grid, s); break;
+    case 2: launch_adjoint_lmn<VisT, P, 2>(fa, grid, s); break;
+    case 4: launch_adjoint_lmn<VisT, P, 4>(fa, grid, s); break;
+    default: launch_adjoint_lmn<VisT, P, 8>(fa, grid, s); break;
+  }
   adjoint_lmn_reduce<<<(3 * D + 3) / 4, 128, 0, s>>>(fa.a.partial, nblk, D, d_grad_lmn);
   if (a.gvis) {
     adjoint_split_g<<<(nbl + 127) / 128, 128, 0, s>>>(a.gavg, nbl, D, const_cast<int4*>(fa.g), const_cast<int16_t*>(fa.gexp));

@@ -29,41 +29,71 @@ int dispatch_pols(const RotateArgs& a, dim3 grid, int precision, cudaStream_t s)
   }
 }
 
-// All-FP64 rotate + average of one item on the integer pipe (kernels_fixed.cuh): the row exponents, then the
-// sums.  nw warps per block take kFxDirs directions each.
+// Blocks of a variant of the fixed-point kernel for the slab plan: as many as an SM runs at a time.  Shared memory (the raw
+// and the split stage, whatever the warps) has room for 3 blocks of 4 pols, 7 of 2 and 11 of 1.  More than kFxWarps warps
+// are not counted, where a kernel's registers allow them: the SM's issue slots are taken by then, and a plan for 5
+// blocks of 4 warps (1 pol) left the last ones of 258 tiles to a few SMs (8 directions: 243 against 279 us).
 template <typename VisT, int P, int NW>
-int launch_fixed_nw(leap_ctx* ctx, const FxArgs& fa, dim3 grid, cudaStream_t s) {
-  constexpr uint32_t bit = 1u << ((sizeof(VisT) == 8 ? 0 : 9) + (P / 2) * 3 + NW / 2);
-  if (!(ctx->fx_attr_set & bit)) {
+int fixed_blocks_nw(leap_ctx* ctx, int& blocks) {
+  int& n = ctx->fx_blocks[sizeof(VisT) == 8 ? 0 : 1][P / 2][NW / 2];
+  if (n == 0) {
     LEAP_CUDA(cudaFuncSetAttribute(rotate_average_fixed<VisT, P, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    fx_smem_bytes<VisT, P>()),
               "set shared memory size");
-    ctx->fx_attr_set |= bit;
+    LEAP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rotate_average_fixed<VisT, P, NW>, NW * 32,
+                                                            fx_smem_bytes<VisT, P>()),
+              "query resident blocks");
+    n = std::max(1, std::min(n, kFxWarps / NW));
   }
-  rotate_average_fixed<VisT, P, NW><<<grid, NW * 32, fx_smem_bytes<VisT, P>(), s>>>(fa);
+  blocks = n;
   return LEAP_OK;
 }
 
 template <typename VisT, int P>
-int launch_fixed(leap_ctx* ctx, const FxArgs& fa, int nw, dim3 grid, cudaStream_t s) {
-  const int64_t elems = fa.r.rows * P;
-  fx_exponents<VisT><<<static_cast<unsigned>((elems + 31) / 32), 256, 0, s>>>(
-      static_cast<const VisT*>(fa.r.vis), elems, fa.r.channels, const_cast<int16_t*>(fa.vexp));
-  switch (nw) {
-    case 1: return launch_fixed_nw<VisT, P, 1>(ctx, fa, grid, s);
-    case 2: return launch_fixed_nw<VisT, P, 2>(ctx, fa, grid, s);
-    default: return launch_fixed_nw<VisT, P, 4>(ctx, fa, grid, s);
+int fixed_blocks_pols(leap_ctx* ctx, int nw, int& blocks) {
+  if constexpr (P < 4) {
+    if (nw == 1) return fixed_blocks_nw<VisT, P, 1>(ctx, blocks);
   }
+  return nw == 2 ? fixed_blocks_nw<VisT, P, 2>(ctx, blocks) : fixed_blocks_nw<VisT, P, 4>(ctx, blocks);
 }
 
-int dispatch_fixed(leap_ctx* ctx, int32_t vis_type, const FxArgs& fa, int nw, dim3 grid, cudaStream_t s) {
+int fixed_blocks(leap_ctx* ctx, int32_t vis_type, int pols, int nw, int& blocks) {
   if (vis_type == LEAP_VIS_C64)
-    return fa.r.pols == 1 ? launch_fixed<float2, 1>(ctx, fa, nw, grid, s)
-                          : fa.r.pols == 2 ? launch_fixed<float2, 2>(ctx, fa, nw, grid, s)
-                                           : launch_fixed<float2, 4>(ctx, fa, nw, grid, s);
-  return fa.r.pols == 1 ? launch_fixed<double2, 1>(ctx, fa, nw, grid, s)
-                        : fa.r.pols == 2 ? launch_fixed<double2, 2>(ctx, fa, nw, grid, s)
-                                         : launch_fixed<double2, 4>(ctx, fa, nw, grid, s);
+    return pols == 1 ? fixed_blocks_pols<float2, 1>(ctx, nw, blocks)
+                     : pols == 2 ? fixed_blocks_pols<float2, 2>(ctx, nw, blocks) : fixed_blocks_pols<float2, 4>(ctx, nw, blocks);
+  return pols == 1 ? fixed_blocks_pols<double2, 1>(ctx, nw, blocks)
+                   : pols == 2 ? fixed_blocks_pols<double2, 2>(ctx, nw, blocks) : fixed_blocks_pols<double2, 4>(ctx, nw, blocks);
+}
+
+// All-FP64 rotate + average of one item on the integer pipe (kernels_fixed.cuh): the row exponents, then the
+// sums.  nw warps per block take kFxDirs directions each; 1 only with fewer than 4 pols.  (fixed_blocks has raised the
+// shared-memory size.)
+template <typename VisT, int P>
+void launch_fixed(const FxArgs& fa, int nw, dim3 grid, cudaStream_t s) {
+  const int64_t elems = fa.r.rows * P;
+  constexpr int smem = fx_smem_bytes<VisT, P>();
+  fx_exponents<VisT><<<static_cast<unsigned>((elems + 31) / 32), 256, 0, s>>>(
+      static_cast<const VisT*>(fa.r.vis), elems, fa.r.channels, const_cast<int16_t*>(fa.vexp));
+  if constexpr (P < 4) {
+    if (nw == 1) {
+      rotate_average_fixed<VisT, P, 1><<<grid, 32, smem, s>>>(fa);
+      return;
+    }
+  }
+  if (nw == 2) rotate_average_fixed<VisT, P, 2><<<grid, 64, smem, s>>>(fa);
+  else rotate_average_fixed<VisT, P, 4><<<grid, 128, smem, s>>>(fa);
+}
+
+void dispatch_fixed(int32_t vis_type, const FxArgs& fa, int nw, dim3 grid, cudaStream_t s) {
+  if (vis_type == LEAP_VIS_C64) {
+    if (fa.r.pols == 1) launch_fixed<float2, 1>(fa, nw, grid, s);
+    else if (fa.r.pols == 2) launch_fixed<float2, 2>(fa, nw, grid, s);
+    else launch_fixed<float2, 4>(fa, nw, grid, s);
+  } else {
+    if (fa.r.pols == 1) launch_fixed<double2, 1>(fa, nw, grid, s);
+    else if (fa.r.pols == 2) launch_fixed<double2, 2>(fa, nw, grid, s);
+    else launch_fixed<double2, 4>(fa, nw, grid, s);
+  }
 }
 
 // The units of an item, `groups` times `nslab` timestep slabs: all slabs cost the same but the last.
@@ -486,23 +516,31 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     const int C = in.channels;
     const bool fixed = precision == LEAP_PRECISION_FP64 && ctx->tab->fx_ok;
     int dirs_per_block = precision == LEAP_PRECISION_FP64 ? 8 : 16;  // 4 warps of 2 or 4 directions
-    int nw = 4;
+    int nw = 4, resident = 1;  // warps per block, blocks per SM
     if (fixed) {
-      // Warps per block: the split of a stage costs a block about as much as one direction, and directions past
-      // the last one are computed for nothing.
-      int64_t best = std::numeric_limits<int64_t>::max();
-      for (int n : {4, 2, 1}) {
-        const int64_t cost = static_cast<int64_t>((w.ndir + n * kFxDirs - 1) / (n * kFxDirs)) * (n * kFxDirs + 1);
-        if (cost < best) {
-          best = cost;
-          nw = n;
-        }
+      // Warps per block.  The split of a stage costs a block about as much as one direction, and directions past the
+      // last one are computed for nothing: cost().  With 4 pols shared memory has room for 3 blocks whatever their warps,
+      // so that fewer warps in a block are fewer on the SM, which costs more than that except for 3 or 4 directions and in
+      // a call without blocks for half of the GPU.  128 antennas, 8 timesteps, 96 channels, us of the kernel with 1, 2 and
+      // 4 warps: 4 pols of complex<float>, 1 direction 399, 367, 311, 4 directions 741, 374, 392, 12 directions 1973, 1008,
+      // 819; 2 pols, 12 directions 734, 500, 577.  36 antennas, 4 timesteps, 48 channels, 4 pols: 12 directions 44 and 50
+      // with 2 and 4 warps, 20 directions 54 and 52.
+      auto groups = [&](int n) { return static_cast<int64_t>((w.ndir + n * kFxDirs - 1) / (n * kFxDirs)); };
+      auto cost = [&](int n) { return groups(n) * (n * kFxDirs + 1); };
+      if (P < 4) {
+        for (int n : {2, 1})
+          if (cost(n) < cost(nw)) nw = n;
+      } else if (w.ndir > 2 && cost(2) < cost(4)) {
+        const bool half_full = 2 * tiles * groups(4) * T >= 3 * static_cast<int64_t>(ctx->sms);
+        if (w.ndir <= 4 || !half_full) nw = 2;
       }
+      if (const int rc = fixed_blocks(ctx, in.vis_type, P, nw, resident)) return rc;
       dirs_per_block = nw * kFxDirs;
     }
     const int dgroups = (w.ndir + dirs_per_block - 1) / dirs_per_block;
     int t_per, c_per, nts, ncs;
-    if (fixed) choose_fixed_slabs(T, C, static_cast<int64_t>(tiles) * dgroups, ctx->sms * (kFxWarps / nw), t_per, c_per, nts, ncs);
+    if (fixed) choose_fixed_slabs(T, C, static_cast<int64_t>(tiles) * dgroups, static_cast<int64_t>(ctx->sms) * resident, t_per, c_per, nts,
+                                  ncs);
     else choose_slabs(T, C, static_cast<int64_t>(tiles) * dgroups, t_per, c_per, nts, ncs);
     const int nslab = nts * ncs;
     const int64_t n = static_cast<int64_t>(w.ndir) * P * nbl;
@@ -532,8 +570,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     if (fixed) {
       LEAP_CUDA(ctx->fx_exp.ensure(sizeof(int16_t) * in.rows * P), "alloc row exponents");
       FxArgs fa{ra, ctx->tab->fx_sp, ctx->fx_tab.as<int4>(), ctx->tab->fx_rho.as<int32_t>(), ctx->fx_exp.as<int16_t>()};
-      const int rc = dispatch_fixed(ctx, in.vis_type, fa, nw, dim3(tiles * dgroups, nslab), s);
-      if (rc != LEAP_OK) return rc;
+      dispatch_fixed(in.vis_type, fa, nw, dim3(tiles * dgroups, nslab), s);
       ++kernels;
     } else {
       const dim3 grid(tiles, dgroups, nslab);

@@ -188,7 +188,8 @@ struct leap_ctx {
   int last_ndir = 0, last_pols = 0, last_nbl = 0;
   // Fixed-point phasors of the all-FP64 form: tables, and the row exponents of the item being rotated.
   DeviceBuffer fx_tab, fx_exp;
-  uint32_t fx_attr_set = 0;           // bit per kernel variant whose shared-memory size was raised
+  int fx_blocks[2][3][3] = {};        // blocks per SM of each kernel variant (0: not asked yet)
+  int adj_blocks[2][3][4] = {};
   // Ring of (start, after rotate, end) events, one triple per recorded call.
   static constexpr int kRing = 256;
   cudaEvent_t ring[kRing][3] = {};
