@@ -472,6 +472,18 @@ bool fx_spectrum(double f0, double df, int32_t channels, const double* lambda, F
   return true;
 }
 
+void spectrum_tables(double f0, double df, int32_t channels, Spectrum& t) {
+  t.lambda.resize(2 * static_cast<size_t>(channels));
+  for (int32_t c = 0; c < channels; ++c) {
+    volatile double prod = static_cast<double>(c) * df;
+    const double lam = 299792458.0 / (f0 + prod);
+    t.lambda[c] = lam;
+    t.lambda[channels + c] = 1.0 / lam;
+  }
+  t.rho.resize(channels);
+  t.fx_ok = fx_spectrum(f0, df, channels, t.lambda.data(), t.sp, t.rho.data());
+}
+
 // cos and sin of the angle x 2^-64 rad, x < 2^64 * pi / 4, in 60-bit fixed point: their Taylor series in whole
 // numbers, each term to 2^-64: the same on every host (long double is software on aarch64: 1.4 ms a context).
 static void fx_cos_sin(uint64_t x, int64_t& c, int64_t& s) {

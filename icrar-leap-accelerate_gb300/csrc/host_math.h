@@ -57,6 +57,40 @@ std::vector<double> es_kernel_transform(int32_t taps, double beta, int32_t n, in
 // a frequency that is not positive and finite, or wavelengths too far from their own formula.
 bool fx_spectrum(double f0, double df, int32_t channels, const double* lambda, FxSpectrum& sp, int32_t* rho);
 
+// Channel wavelengths of a spectral window and their reciprocals, and its fixed-point form: the host's copy of what the
+// kernels read.
+struct Spectrum {
+  int32_t channels = 0;               // 0: the device tables hold nothing to rely on
+  double f0 = 0.0, df = 0.0;
+  std::vector<double> lambda;         // [wavelengths][their reciprocals]
+  std::vector<int32_t> rho;           // corrections of the fixed-point phasors
+  FxSpectrum sp{};
+  bool fx_ok = false;                 // the fixed-point phasors apply to this window
+};
+
+// Wavelengths c / (f0 + ch*df) with each operation rounded on its own, as the reference's
+// Constants::GetChannelWavelength (no fused multiply-add), and the rest of `t`.
+void spectrum_tables(double f0, double df, int32_t channels, Spectrum& t);
+
+// Makes `t` and the device tables those of a window: reserve() allocates them for `channels` channels, upload() copies
+// them; both return 0 or an error, which leaves `t` empty, so that the next call starts over.
+template <typename Reserve, typename Upload>
+int update_spectrum(Spectrum& t, double f0, double df, int32_t channels, Reserve reserve, Upload upload) {
+  if (channels > 0 && t.channels == channels && t.f0 == f0 && t.df == df) return 0;
+  t.channels = 0;
+  t.fx_ok = false;
+  if (const int rc = reserve()) return rc;
+  spectrum_tables(f0, df, channels, t);
+  if (const int rc = upload()) {
+    t.fx_ok = false;
+    return rc;
+  }
+  t.channels = channels;
+  t.f0 = f0;
+  t.df = df;
+  return 0;
+}
+
 // The two phasor tables: kFxTable entries exp(2 pi i j / 2^10), then kFxTable of exp(2 pi i j / 2^20).
 void fx_tables(std::vector<FxLimbs>& out);
 

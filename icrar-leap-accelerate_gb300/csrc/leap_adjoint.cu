@@ -139,19 +139,19 @@ int32_t leap_backward(leap_ctx* ctx, int32_t slot, const double* d_dd, int32_t n
   // aligned to that, and spectral windows that fixed_phase.h does not take, use the FP64 ones.
   const size_t esz = aa.vis_c64 ? sizeof(float2) : sizeof(double2);
   const uintptr_t align = esz * aa.P % 16 == 0 ? 16 : 8;
-  if (ctx->tab->fx_ok && in.rows % nbl == 0 && (reinterpret_cast<uintptr_t>(aa.vis) | reinterpret_cast<uintptr_t>(d_grad_vis)) % align == 0) {
+  if (ctx->tab->spectrum.fx_ok && in.rows % nbl == 0 && (reinterpret_cast<uintptr_t>(aa.vis) | reinterpret_cast<uintptr_t>(d_grad_vis)) % align == 0) {
     LEAP_CUDA(ctx->fx_exp.ensure(sizeof(int16_t) * in.rows), "alloc row exponents");
     LEAP_CUDA(ctx->adj_g.ensure(sizeof(int4) * 2 * static_cast<size_t>(nbl) * D), "alloc adjoint scratch");
     LEAP_CUDA(ctx->adj_gexp.ensure(sizeof(int16_t) * nbl), "alloc adjoint scratch");
     AdjointFixedArgs fa{};
     fa.a = aa;
-    fa.sp = ctx->tab->fx_sp;
+    fa.sp = ctx->tab->spectrum.sp;
     fa.tab = ctx->fx_tab.as<int4>();
     fa.rho = ctx->tab->fx_rho.as<int32_t>();
     fa.lambda = ctx->tab->lambda.as<double>();
-    fa.inv_lambda = ctx->tab->lambda.as<double>() + ctx->tab->lambda_host.size() / 2;
+    fa.inv_lambda = ctx->tab->lambda.as<double>() + ctx->tab->spectrum.channels;
     fa.vexp = ctx->fx_exp.as<int16_t>();
-    fa.kexp = std::ilogb(ctx->tab->fx_sp.kmax) + 1;
+    fa.kexp = std::ilogb(ctx->tab->spectrum.sp.kmax) + 1;
     fa.T = static_cast<int>(in.rows / nbl);
     fa.g = ctx->adj_g.as<int4>();
     fa.gexp = ctx->adj_gexp.as<int16_t>();

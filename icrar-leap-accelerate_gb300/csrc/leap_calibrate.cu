@@ -317,38 +317,27 @@ int launch_pipe(leap_ctx* ctx, const PipeParams& pp, int grid, cudaStream_t s) {
   return LEAP_OK;
 }
 
-// Channel wavelengths of at least `channels` channels, computed exactly as Constants::GetChannelWavelength does, and
-// the fixed-point spectral window; uploaded only when the channel count or the spectral window changes.
+// Channel wavelengths and the fixed-point spectral window of `channels` channels; uploaded only when the channel count or
+// the spectral window changes.
 int ensure_spectrum(leap_ctx* ctx, int channels, cudaStream_t s) {
-  const Metadata& md = ctx->md;
-  LEAP_CUDA(ctx->tab->lambda.ensure(sizeof(double) * 2 * channels), "alloc wavelengths");
-  if (ctx->tab->lambda_host.size() != static_cast<size_t>(2 * channels) || ctx->tab->lambda_f0 != md.k.freq_start_hz ||
-      ctx->tab->lambda_df != md.k.freq_inc_hz) {
-    // [wavelengths][their reciprocals]: c / (f0 + ch*df) with each operation rounded on its own,
-    // as the reference's Constants::GetChannelWavelength (no fused multiply-add).
-    ctx->tab->lambda_host.resize(2 * channels);
-    for (int c = 0; c < channels; ++c) {
-      volatile double prod = static_cast<double>(c) * md.k.freq_inc_hz;
-      const double lam = kSpeedOfLight / (md.k.freq_start_hz + prod);
-      ctx->tab->lambda_host[c] = lam;
-      ctx->tab->lambda_host[channels + c] = 1.0 / lam;
-    }
-    ctx->tab->lambda_f0 = md.k.freq_start_hz;
-    ctx->tab->lambda_df = md.k.freq_inc_hz;
-    LEAP_CUDA(cudaMemcpyAsync(ctx->tab->lambda.ptr, ctx->tab->lambda_host.data(), sizeof(double) * 2 * channels,
-                              cudaMemcpyHostToDevice, s),
-              "upload wavelengths");
-    ctx->tab->fx_rho_host.resize(channels);
-    ctx->tab->fx_ok = fx_spectrum(md.k.freq_start_hz, md.k.freq_inc_hz, channels, ctx->tab->lambda_host.data(), ctx->tab->fx_sp,
-                             ctx->tab->fx_rho_host.data());
-    if (ctx->tab->fx_ok) {
-      LEAP_CUDA(ctx->tab->fx_rho.ensure(sizeof(int32_t) * channels), "alloc wavelength corrections");
-      LEAP_CUDA(cudaMemcpyAsync(ctx->tab->fx_rho.ptr, ctx->tab->fx_rho_host.data(), sizeof(int32_t) * channels,
-                                cudaMemcpyHostToDevice, s),
-                "upload wavelength corrections");
-    }
-  }
-  return LEAP_OK;
+  LaunchTables& tab = *ctx->tab;
+  return update_spectrum(
+      tab.spectrum, ctx->md.k.freq_start_hz, ctx->md.k.freq_inc_hz, channels,
+      [&]() -> int {
+        LEAP_CUDA(tab.lambda.ensure(sizeof(double) * 2 * channels), "alloc wavelengths");
+        LEAP_CUDA(tab.fx_rho.ensure(sizeof(int32_t) * channels), "alloc wavelength corrections");
+        return LEAP_OK;
+      },
+      [&]() -> int {
+        LEAP_CUDA(cudaMemcpyAsync(tab.lambda.ptr, tab.spectrum.lambda.data(), sizeof(double) * 2 * channels,
+                                  cudaMemcpyHostToDevice, s),
+                  "upload wavelengths");
+        if (tab.spectrum.fx_ok)
+          LEAP_CUDA(cudaMemcpyAsync(tab.fx_rho.ptr, tab.spectrum.rho.data(), sizeof(int32_t) * channels,
+                                    cudaMemcpyHostToDevice, s),
+                    "upload wavelength corrections");
+        return LEAP_OK;
+      });
 }
 
 // Rotate + average of every item into ctx->avg ([D][P][nbl]).
@@ -514,7 +503,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     Integration& in = ctx->integ.at(w.slot);
     const int T = static_cast<int>(in.rows / nbl);
     const int C = in.channels;
-    const bool fixed = precision == LEAP_PRECISION_FP64 && ctx->tab->fx_ok;
+    const bool fixed = precision == LEAP_PRECISION_FP64 && ctx->tab->spectrum.fx_ok;
     int dirs_per_block = precision == LEAP_PRECISION_FP64 ? 8 : 16;  // 4 warps of 2 or 4 directions
     int nw = 4, resident = 1;  // warps per block, blocks per SM
     if (fixed) {
@@ -550,7 +539,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     ra.uvw = in.uvw.as<double>();
     ra.dd = d_dd + 9 * static_cast<int64_t>(w.dir0);
     ra.lambda = ctx->tab->lambda.as<double>();
-    ra.inv_lambda = ctx->tab->lambda.as<double>() + ctx->tab->lambda_host.size() / 2;
+    ra.inv_lambda = ctx->tab->lambda.as<double>() + ctx->tab->spectrum.channels;
     ra.twiddle = ctx->twiddle.as<float2>();
     ra.rows = in.rows;
     ra.channels = C;
@@ -569,7 +558,7 @@ int rotate_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
     ra.err = ctx->dev_err.as<int>();
     if (fixed) {
       LEAP_CUDA(ctx->fx_exp.ensure(sizeof(int16_t) * in.rows * P), "alloc row exponents");
-      FxArgs fa{ra, ctx->tab->fx_sp, ctx->fx_tab.as<int4>(), ctx->tab->fx_rho.as<int32_t>(), ctx->fx_exp.as<int16_t>()};
+      FxArgs fa{ra, ctx->tab->spectrum.sp, ctx->fx_tab.as<int4>(), ctx->tab->fx_rho.as<int32_t>(), ctx->fx_exp.as<int16_t>()};
       dispatch_fixed(in.vis_type, fa, nw, dim3(tiles * dgroups, nslab), s);
       ++kernels;
     } else {
@@ -651,7 +640,7 @@ int refant_stage(leap_ctx* ctx, const std::vector<WorkItem>& items, const double
       rr.uvw = in.uvw.as<double>();
       rr.dd = d_dd + 9 * static_cast<int64_t>(w.dir0);
       rr.lambda = ctx->tab->lambda.as<double>();
-      rr.inv_lambda = ctx->tab->lambda.as<double>() + ctx->tab->lambda_host.size() / 2;
+      rr.inv_lambda = ctx->tab->lambda.as<double>() + ctx->tab->spectrum.channels;
       rr.rows = in.rows;
       rr.channels = in.channels;
       rr.pols = in.pols;

@@ -117,11 +117,7 @@ struct TuneChoice {
 struct LaunchTables {
   DeviceBuffer pipe_items, pipe_order, grid_items, grid_order, reduce_items, refant_items, refant_reduce;
   DeviceBuffer lambda, fx_rho;        // wavelengths and their reciprocals; corrections of the fixed-point phasors
-  std::vector<double> lambda_host;
-  double lambda_f0 = 0.0, lambda_df = 0.0;
-  std::vector<int32_t> fx_rho_host;
-  FxSpectrum fx_sp{};
-  bool fx_ok = false;                 // the fixed-point phasors apply to this window
+  Spectrum spectrum;
   void release() {
     for (DeviceBuffer* b : {&pipe_items, &pipe_order, &grid_items, &grid_order, &reduce_items, &refant_items,
                             &refant_reduce, &lambda, &fx_rho})
