@@ -43,12 +43,15 @@ struct FxArgs {
   const int16_t* vexp;    // [rows][pols]: the largest component of the row is below 2^vexp
 };
 
-// A component's magnitude by its bits (the high word of a double): ordered as the magnitudes are, NaN above all.
+// A component's magnitude by its bits (the high word of a double, whose lowest bit also tells a low word that is not 0 from
+// an exact zero): ordered as the magnitudes are, NaN above all.
 __device__ __forceinline__ uint32_t fx_magnitude(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
-__device__ __forceinline__ uint32_t fx_magnitude(double x) { return static_cast<uint32_t>(__double2hiint(x)) & 0x7FFFFFFFu; }
+__device__ __forceinline__ uint32_t fx_magnitude(double x) {
+  return (static_cast<uint32_t>(__double2hiint(x)) & 0x7FFFFFFFu) | (__double2loint(x) != 0 ? 1u : 0u);
+}
 
 // Exponent of the largest magnitude m: it is below 2^e.  kFxPlain where the integer sums do not apply.  m == 0: a
-// row of zeros (or of doubles below 2^-1042), which adds nothing.
+// row of zeros, which adds nothing.
 template <typename VisT>
 __device__ __forceinline__ int16_t fx_exponent(uint32_t m) {
   int e;
