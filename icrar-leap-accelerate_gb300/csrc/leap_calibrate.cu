@@ -979,15 +979,18 @@ int autotune_batch(leap_ctx* ctx, const std::vector<WorkItem>& items, int32_t D,
 }
 
 // Everything that a recorded batched call has fixed besides buffer addresses: its launches and tables follow from the
-// key, the metadata, and the shape of each slot.  Empty where a slot is not set (the call is refused).
-std::string graph_signature(const leap_ctx* ctx, const std::vector<WorkItem>& items, const std::string& key) {
-  std::string k = key + "|md" + std::to_string(ctx->md_gen);
+// items, the options of batch_key, the metadata, and the shape of each slot.  Empty where a slot is not set (the call
+// is refused).
+std::vector<int64_t> graph_signature(const leap_ctx* ctx, const std::vector<WorkItem>& items, int32_t D, int32_t precision) {
+  std::vector<int64_t> k;
+  k.reserve(7 + 8 * items.size());
+  k.insert(k.end(), {static_cast<int64_t>(ctx->md_gen), D, precision, ctx->tc_gemm, ctx->mma_rotate, ctx->gridded,
+                     ctx->grid_shared_groups});
   for (const auto& w : items) {
     auto it = ctx->integ.find(w.slot);
     if (it == ctx->integ.end()) return {};
     const Integration& in = it->second;
-    k += "|" + std::to_string(in.rows) + "," + std::to_string(in.channels) + "," + std::to_string(in.pols) + "," +
-         std::to_string(in.vis_type) + (in.has_map ? "m" : "");
+    k.insert(k.end(), {w.slot, w.dir0, w.ndir, in.rows, in.channels, in.pols, in.vis_type, in.has_map});
   }
   return k;
 }
@@ -1022,9 +1025,8 @@ int calibrate_batched_impl(leap_ctx* ctx, const leap_work_item* witems, int32_t 
   if (!witems || nitems <= 0) return fail(ctx, LEAP_ERR_INVALID_ARGUMENT, "no work items");
   std::vector<WorkItem> items(nitems);
   for (int i = 0; i < nitems; ++i) items[i] = WorkItem{witems[i].slot, witems[i].first_direction, witems[i].ndirections};
-  const std::string key = batch_key(ctx, items, D, precision);
   cudaStream_t s = ctx->stream;
-  const std::string sig = graph_signature(ctx, items, key);
+  const std::vector<int64_t> sig = graph_signature(ctx, items, D, precision);
   if (ctx->graph_replay && !sig.empty() && ctx->graph_sig == sig) {
     bool done = false;
     const int rc = replay_batched(ctx, items, D, precision, done);
@@ -1037,6 +1039,7 @@ int calibrate_batched_impl(leap_ctx* ctx, const leap_work_item* witems, int32_t 
     explicit OwnTables(leap_ctx* c) : ctx(c) { ctx->tab = &ctx->batched; }
     ~OwnTables() { ctx->tab = &ctx->single; }
   } own(ctx);
+  const std::string key = batch_key(ctx, items, D, precision);
   auto t = ctx->tuned.find(key);
   if (t != ctx->tuned.end()) {
     ctx->tune = t->second;

@@ -11,7 +11,6 @@
 #include <cstring>
 #include <limits>
 #include <map>
-#include <queue>
 #include <memory>
 #include <string>
 #include <vector>
@@ -159,7 +158,7 @@ struct leap_ctx {
   cudaEvent_t stage_done[2] = {nullptr, nullptr};
   std::map<std::string, TuneChoice> tuned;
   // The recorded batched call: replayed for calls of the same signature (graph_signature) while no buffer moves.
-  std::string graph_sig;              // empty: nothing to replay
+  std::vector<int64_t> graph_sig;     // empty: nothing to replay
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_epoch = 0;
   int graph_kernels = 0;
