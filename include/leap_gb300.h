@@ -200,8 +200,9 @@ int32_t leap_calibrate_async(leap_ctx* ctx, int32_t slot, const double* d_dd, in
  * ndirections row-major 3x3 matrices (HOST), items[i] selects
  * dd[first_direction .. first_direction + ndirections); cal_out (HOST) is
  * [ndirections][S].  The first call of a new shape tunes the launch plan (see
- * leap_set_autotune) and records the launches as a CUDA graph, which later
- * calls of the same shape replay. */
+ * leap_set_autotune) and records the launches as a CUDA graph.  Later calls of
+ * the same items replay it on what their slots hold then, while the metadata,
+ * the options and the slots' shapes stay as they were. */
 int32_t leap_calibrate_batched(leap_ctx* ctx, const leap_work_item* items, int32_t nitems, const double* dd,
                                int32_t ndirections, int32_t precision, double* cal_out);
 
@@ -249,7 +250,7 @@ int32_t leap_get_avgdata(leap_ctx* ctx, int32_t direction, double* out);
  * reference-antenna rows hold the compensated sums the solve used. */
 int32_t leap_get_avgdata_device(leap_ctx* ctx, int32_t pol, double* d_out, void* stream);
 
-/* Adjoint of one calibrate call (rotate -> average -> arg -> solve), in FP64.
+/* Adjoint of one calibrate call (rotate -> average -> arg -> solve), to FP64 accuracy.
  * Replaces nothing in the reference (its path has no gradient); it is the
  * backward of the differentiable form for the Python leap_drops layer.
  * Inputs (DEVICE, on `stream`; NULL: the context's stream):
